@@ -9,19 +9,23 @@ namespace {
 constexpr int kBatchThreads = 256;
 
 // NIP of every product i: sum over its rows r in [row_off[i], row_off[i+1])
-// of A of sum_{k in A(r,:)} len(B(k,:)).  One CTA per product.
+// of A of sum_{k in A(r,:)} len(B(k,:)).  gridDim.y CTAs per product, each
+// with every gridDim.y-th slice of its entries, adding to nip[i] (zeroed by
+// the caller): few large products still fill the chip.
 __global__ __launch_bounds__(kBatchThreads) void k_product_nip(
     const int32_t* __restrict__ a_rpt, const int32_t* __restrict__ a_col,
     const int32_t* __restrict__ b_rpt, const int32_t* __restrict__ row_off,
-    long long* __restrict__ nip) {
+    unsigned long long* __restrict__ nip) {
     __shared__ long long s_part[kBatchThreads / kWarp];
     const int i = blockIdx.x;
     const int r0 = row_off[i];
     const int r1 = row_off[i + 1];
     const int e0 = a_rpt[r0];
     const int e1 = a_rpt[r1];
+    const long long stride = static_cast<long long>(gridDim.y) * kBatchThreads;
     long long s = 0;
-    for (int e = e0 + threadIdx.x; e < e1; e += kBatchThreads) {
+    for (long long e = e0 + static_cast<long long>(blockIdx.y) * kBatchThreads + threadIdx.x;
+         e < e1; e += stride) {
         const int c = __ldg(a_col + e);
         s += __ldg(b_rpt + c + 1) - __ldg(b_rpt + c);
     }
@@ -32,32 +36,103 @@ __global__ __launch_bounds__(kBatchThreads) void k_product_nip(
     if (threadIdx.x == 0) {
         long long t = 0;
         for (int w = 0; w < kBatchThreads / kWarp; w++) t += s_part[w];
-        nip[i] = t;
+        if (t != 0) atomicAdd(nip + i, static_cast<unsigned long long>(t));
     }
 }
 
-// Split a group's C into per-product CSR: for product i (rows [r0, r1) of the
-// group's C, local row 0 at r0), write its own row pointer starting at 0 into
-// rpt_out + out_off[i] and shift its columns back to local indices.
+// Split a group's C into per-product CSR: product i (rows [r0, r1) of the
+// group's C, local row 0 at r0) gets its own row pointer starting at 0 in
+// rpt_out + out_off[i], and its columns are shifted back to local indices in
+// place.  Bound by memory: C.col is read and written once, so the work is cut
+// by entries and rows, not by products (one CTA per product left 20 products
+// of 1.4 M entries on 20 SMs: 4.9 ms; by entries 0.04 ms).  The first row_ctas
+// CTAs take kUnpackRows rows each, the others kUnpackEntries entries each; a
+// CTA finds its first product by a 32-way search.
+constexpr int kUnpackRows = 2048;
+constexpr int kUnpackEntries = 4096;
+
+// The last i in [lo, hi) with start(i) <= x, by one warp (start(lo) <= x).
+template<typename F>
+__device__ __forceinline__ int warp_last_le(int lo, int hi, int x, F&& start) {
+    const int lane = threadIdx.x & 31;
+    while (hi - lo > 1) {  // uniform over the warp
+        const int step = (hi - lo + kWarp - 1) / kWarp;
+        const long long at = lo + static_cast<long long>(lane) * step;
+        const unsigned le = __ballot_sync(0xffffffffu, at < hi && start(static_cast<int>(at)) <= x);
+        lo += (31 - __clz(le)) * step;
+        hi = min(lo + step, hi);
+    }
+    return lo;
+}
+
 __global__ __launch_bounds__(kBatchThreads) void k_unpack(
     const int32_t* __restrict__ c_rpt, int32_t* __restrict__ c_col,
     const int32_t* __restrict__ row_off, const int32_t* __restrict__ col_off,
-    const int64_t* __restrict__ out_off, int32_t first, int32_t* __restrict__ rpt_out,
-    int32_t* __restrict__ pos_out) {
-    const int i = first + blockIdx.x;  // product index in the batch
+    const int64_t* __restrict__ out_off, int32_t first, int32_t count, int32_t row_ctas,
+    int32_t nnz, int32_t* __restrict__ rpt_out, int32_t* __restrict__ pos_out) {
+    __shared__ int32_t s_first;
+    const int tid = threadIdx.x;
+    const int last = first + count;
     const int base_row = row_off[first];
-    const int r0 = row_off[i] - base_row;
-    const int r1 = row_off[i + 1] - base_row;
-    const int p0 = c_rpt[r0];
-    const int p1 = c_rpt[r1];
-    if (threadIdx.x == 0) {
-        pos_out[2 * i] = p0;
-        pos_out[2 * i + 1] = p1 - p0;
+    const int rows = row_off[last] - base_row;
+    auto entry_start = [&](int i) { return c_rpt[row_off[i] - base_row]; };
+    if (static_cast<int>(blockIdx.x) < row_ctas) {
+        // per product: its place in C and its row pointer's last word
+        for (int i = first + blockIdx.x * kBatchThreads + tid; i < last;
+             i += row_ctas * kBatchThreads) {
+            const int p0 = entry_start(i);
+            const int n = entry_start(i + 1) - p0;
+            pos_out[2 * i] = p0;
+            pos_out[2 * i + 1] = n;
+            rpt_out[out_off[i] + (row_off[i + 1] - row_off[i])] = n;
+        }
+        const int t0 = blockIdx.x * kUnpackRows;
+        const int t1 = rows - t0 < kUnpackRows ? rows : t0 + kUnpackRows;
+        if (t0 >= t1) return;  // uniform over the CTA
+        if (tid < kWarp) {
+            const int i = warp_last_le(first, last, base_row + t0,
+                                       [&](int k) { return row_off[k]; });
+            if (tid == 0) s_first = i;
+        }
+        __syncthreads();
+        int i = s_first;
+        for (int t = t0 + tid; t < t1; t += kBatchThreads) {
+            while (row_off[i + 1] - base_row <= t) i++;  // empty products are passed over
+            rpt_out[out_off[i] + (t - (row_off[i] - base_row))] = c_rpt[t] - entry_start(i);
+        }
+        return;
     }
-    int32_t* out = rpt_out + out_off[i];
-    for (int t = threadIdx.x; t <= r1 - r0; t += kBatchThreads) out[t] = c_rpt[r0 + t] - p0;
-    const int shift = col_off[i];
-    for (int p = p0 + threadIdx.x; p < p1; p += kBatchThreads) c_col[p] -= shift;
+    const int p0 = (blockIdx.x - row_ctas) * kUnpackEntries;
+    const int p1 = nnz - p0 < kUnpackEntries ? nnz : p0 + kUnpackEntries;
+    if (tid < kWarp) {
+        const int i = warp_last_le(first, last, p0, entry_start);
+        if (tid == 0) s_first = i;
+    }
+    __syncthreads();
+    int i = s_first;
+    int end = entry_start(i + 1);
+    int shift = col_off[i];
+    if (end >= p1 && p1 - p0 == kUnpackEntries) {  // one product, a whole chunk: 16 bytes a load
+        int4* c4 = reinterpret_cast<int4*>(c_col + p0);
+#pragma unroll
+        for (int k = 0; k < kUnpackEntries / 4 / kBatchThreads; k++) {
+            int4 v = c4[k * kBatchThreads + tid];
+            v.x -= shift;
+            v.y -= shift;
+            v.z -= shift;
+            v.w -= shift;
+            c4[k * kBatchThreads + tid] = v;
+        }
+        return;
+    }
+    for (long long p = p0 + tid; p < p1; p += kBatchThreads) {
+        if (end <= p) {
+            while (entry_start(i + 1) <= p) i++;
+            end = entry_start(i + 1);
+            shift = col_off[i];
+        }
+        c_col[p] -= shift;
+    }
 }
 
 // NIP of many independent pairs (A_i, B_i) in one launch: pair i's A entries
@@ -115,16 +190,27 @@ cudaError_t launch_product_nip(const int32_t* a_rpt, const int32_t* a_col, const
                                const int32_t* row_off, int32_t count, long long* nip,
                                cudaStream_t s) {
     if (count <= 0) return cudaSuccess;
-    k_product_nip<<<count, kBatchThreads, 0, s>>>(a_rpt, a_col, b_rpt, row_off, nip);
+    if (cudaError_t e = cudaMemsetAsync(nip, 0, sizeof(long long) * static_cast<size_t>(count), s);
+        e != cudaSuccess)
+        return e;
+    // about eight CTAs per SM over all products
+    const int per = 148 * 8 / count;
+    const dim3 grid(count, per < 1 ? 1 : per > 64 ? 64 : per);
+    k_product_nip<<<grid, kBatchThreads, 0, s>>>(a_rpt, a_col, b_rpt, row_off,
+                                                 reinterpret_cast<unsigned long long*>(nip));
     return cudaGetLastError();
 }
 
 cudaError_t launch_unpack(const int32_t* c_rpt, int32_t* c_col, const int32_t* row_off,
                           const int32_t* col_off, const int64_t* out_off, int32_t first,
-                          int32_t count, int32_t* rpt_out, int32_t* pos_out, cudaStream_t s) {
+                          int32_t count, int32_t rows, int32_t nnz, int32_t* rpt_out,
+                          int32_t* pos_out, cudaStream_t s) {
     if (count <= 0) return cudaSuccess;
-    k_unpack<<<count, kBatchThreads, 0, s>>>(c_rpt, c_col, row_off, col_off, out_off, first,
-                                             rpt_out, pos_out);
+    const int row_ctas = rows > 0 ? (rows - 1) / kUnpackRows + 1 : 1;
+    const int col_ctas = nnz > 0 ? (nnz - 1) / kUnpackEntries + 1 : 0;
+    k_unpack<<<row_ctas + col_ctas, kBatchThreads, 0, s>>>(c_rpt, c_col, row_off, col_off, out_off,
+                                                           first, count, row_ctas, nnz, rpt_out,
+                                                           pos_out);
     return cudaGetLastError();
 }
 

@@ -230,7 +230,8 @@ cudaError_t launch_product_nip(const int32_t* a_rpt, const int32_t* a_col, const
                                cudaStream_t s);
 cudaError_t launch_unpack(const int32_t* c_rpt, int32_t* c_col, const int32_t* row_off,
                           const int32_t* col_off, const int64_t* out_off, int32_t first,
-                          int32_t count, int32_t* rpt_out, int32_t* pos_out, cudaStream_t s);
+                          int32_t count, int32_t rows, int32_t nnz, int32_t* rpt_out,
+                          int32_t* pos_out, cudaStream_t s);
 // CSR transpose (k_transpose.cu): row-sort ladder (key = length of a row of
 // A^T), column counts, and the keyed scatter.
 int transpose_ladder_f64(const BinLauncher** out);

@@ -1355,8 +1355,8 @@ spgemm_status batch(spgemm_handle_s* h, const spgemm_batch_desc* d, const spgemm
         if (Cg.col) blocks.push_back(Cg.col);
         if (Cg.val) blocks.push_back(Cg.val);
         if (plan == nullptr) {
-            e = launch_unpack(Cg.rpt, Cg.col, d_row, d_col, d_off, p0, p1 - p0, rpt_out, d_pos,
-                              stream);
+            e = launch_unpack(Cg.rpt, Cg.col, d_row, d_col, d_off, p0, p1 - p0, r1 - r0, Cg.nnz,
+                              rpt_out, d_pos, stream);
             if (e == cudaSuccess) e = cudaFreeAsync(Cg.rpt, stream);  // split copies what it needs
         } else {
             // the group's fill graph, then its split, as two nodes of the plan
@@ -1364,8 +1364,8 @@ spgemm_status batch(spgemm_handle_s* h, const spgemm_batch_desc* d, const spgemm
             cudaGraph_t split = nullptr;
             e = cudaStreamBeginCapture(plan->capture, cudaStreamCaptureModeThreadLocal);
             if (e == cudaSuccess)
-                e = launch_unpack(Cg.rpt, Cg.col, d_row, d_col, d_off, p0, p1 - p0, rpt_out,
-                                  d_pos, plan->capture);
+                e = launch_unpack(Cg.rpt, Cg.col, d_row, d_col, d_off, p0, p1 - p0, r1 - r0,
+                                  Cg.nnz, rpt_out, d_pos, plan->capture);
             const cudaError_t ee = cudaStreamEndCapture(plan->capture, &split);
             if (e == cudaSuccess) e = ee;
             if (e == cudaSuccess) {
