@@ -3,14 +3,22 @@
 // The reference has no transpose: its Galerkin use (R = P^T for R*A*P) leaves
 // the transpose to the caller.  Here it is a library call so that a chained
 // product stays on the device:
-//   1. column counts of A (warp-aggregated atomics) into T.rpt;
+//   1. column counts of A (warp-aggregated atomics) into T.rpt; the atomic's
+//      old value is the entry's rank in its column, kept per entry (in T.col,
+//      which nothing else needs yet);
 //   2. the product path's binning pass with the scan (k_bin.cu) turns the
 //      counts into T.rpt and bins T's rows by length;
-//   3. scatter: every entry (i, j) of A takes a slot of row j of T through an
-//      atomic cursor and stores the 64-bit key (i << 32 | position in A);
-//   4. per bin, sort each row's keys ascending (the row indices i are unique
-//      within a row, so the order is fully determined) and write T.col = i,
-//      T.val = A.val[position].
+//   3. scatter: entry (i, j) of A at position e goes to place T.rpt[j] + rank
+//      as one 16-byte record: the key (i << 32 | e) and the value;
+//   4. each row's records are put in key order (the keys are unique, so the
+//      order is fully determined) and written as T.col = i, T.val: rows of up
+//      to kTrFlat entries by counting, per record, the row's smaller keys;
+//      longer rows by sorting.
+// Bound by random 32-byte sectors: one atomic and one record write per entry,
+// whatever the record's size up to 32 bytes, so the value travels with the key
+// instead of being gathered after the sort.  Entries are dealt to lanes flat
+// (a warp per row of A left most lanes idle at 5.5 entries a row, and took a
+// second atomic per entry).
 // Sorting uses the bitonic network in which every comparator sends the
 // smaller key to the lower index; a row of len keys runs the network of the
 // next power of two with the missing tail taken as +infinity, and every
@@ -22,20 +30,29 @@ namespace b200 {
 
 namespace {
 
-constexpr uint64_t kKeyInf = ~0ull;
+// One entry on its way to its row of T: key = row of A << 32 | position in A,
+// val = the bits of the value.
+struct __align__(16) TrRec {
+    uint64_t key;
+    uint64_t val;
+};
 
-__device__ __forceinline__ void cas_asc(uint64_t* a, long long lo, long long hi) {
-    const uint64_t x = a[lo];
-    const uint64_t y = a[hi];
-    if (x > y) {
+__device__ __forceinline__ uint64_t sort_key(uint64_t x) { return x; }
+__device__ __forceinline__ uint64_t sort_key(const TrRec& x) { return x.key; }
+
+template<typename T>
+__device__ __forceinline__ void cas_asc(T* a, long long lo, long long hi) {
+    const T x = a[lo];
+    const T y = a[hi];
+    if (sort_key(x) > sort_key(y)) {
         a[lo] = y;
         a[hi] = x;
     }
 }
 
 // Ascending sort of a[0, len) by the CTA (a in shared or global memory).
-template<int THREADS>
-__device__ void cta_sort_keys(uint64_t* a, long long len) {
+template<int THREADS, typename T>
+__device__ void cta_sort_keys(T* a, long long len) {
     long long N = 1;
     while (N < len) N <<= 1;
     const long long pairs = N >> 1;
@@ -59,77 +76,191 @@ __device__ void cta_sort_keys(uint64_t* a, long long len) {
     }
 }
 
+__host__ __device__ __forceinline__ const TrRec* recs_of(const ProductArgs& p) {
+    return reinterpret_cast<const TrRec*>(p.keys);
+}
+
+template<typename V>
+__device__ __forceinline__ uint64_t val_bits(V v) {
+    if constexpr (sizeof(V) == 8) return static_cast<uint64_t>(__double_as_longlong(v));
+    else return __float_as_uint(v);
+}
+
+template<typename V>
+__device__ __forceinline__ V val_of(uint64_t bits) {
+    if constexpr (sizeof(V) == 8) return __longlong_as_double(static_cast<long long>(bits));
+    else return __uint_as_float(static_cast<uint32_t>(bits));
+}
+
+// ---- 1. column counts and ranks ---------------------------------------------
+// rank[e] = entry e's place among its column's entries, in the order of the
+// atomics (any order: step 4 sorts).  A column index outside [0, n) is not
+// counted and its rank is -1; the host sees the total fall short of nnz and
+// reports the operand as invalid.  kCountUnroll atomics per lane in flight.
+constexpr int kCountUnroll = 4;
+
+__global__ __launch_bounds__(256) void k_col_count(const int32_t* __restrict__ col, int32_t nnz,
+                                                   int32_t n, int32_t* __restrict__ cnt,
+                                                   int32_t* __restrict__ rank) {
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const long long stride = static_cast<long long>(gridDim.x) * blockDim.x * kCountUnroll;
+    // the loop bound is warp-uniform, so every lane joins each match
+    for (long long base = (static_cast<long long>(blockIdx.x) * blockDim.x +
+                           (threadIdx.x & ~31)) * kCountUnroll;
+         base < nnz; base += stride) {
+        int32_t c[kCountUnroll];
+        int32_t first[kCountUnroll];
+        unsigned peers[kCountUnroll];
+#pragma unroll
+        for (int u = 0; u < kCountUnroll; u++) {
+            const long long e = base + u * kWarp + lane;
+            c[u] = e < nnz ? __ldg(col + e) : -1;
+            if (c[u] >= n) c[u] = -1;
+        }
+#pragma unroll
+        for (int u = 0; u < kCountUnroll; u++) {
+            peers[u] = __match_any_sync(0xffffffffu, c[u]);
+            first[u] = 0;
+            if (c[u] >= 0 && (peers[u] & below) == 0u)
+                first[u] = atomicAdd(cnt + c[u], __popc(peers[u]));
+        }
+#pragma unroll
+        for (int u = 0; u < kCountUnroll; u++) {
+            const long long e = base + u * kWarp + lane;
+            const int r = __shfl_sync(0xffffffffu, first[u], __ffs(peers[u]) - 1) +
+                          __popc(peers[u] & below);
+            if (e < nnz) rank[e] = c[u] >= 0 ? r : -1;
+        }
+    }
+}
+
+// ---- 3. scatter of records --------------------------------------------------
+// A warp takes kScatterTile consecutive entries of A, finds the rows of the
+// first and the last by a 32-way search of A.rpt, and each lane finds its
+// entries' rows by a binary search between them.  Entries whose column is
+// outside [0, n) were not ranked and are skipped.
+constexpr int kScatterPer = 8;
+constexpr int kScatterTile = kWarp * kScatterPer;
+
+// The last r in [0, m) with rpt[r] <= e, by one warp (rpt[0] <= e, m >= 1).
+__device__ __forceinline__ int warp_row_of(const int32_t* __restrict__ rpt, int32_t m, int32_t e) {
+    const int lane = threadIdx.x & 31;
+    int lo = 0;
+    int hi = m;
+    while (hi - lo > 1) {  // uniform over the warp
+        const int step = (hi - lo + kWarp - 1) / kWarp;
+        const long long at = lo + static_cast<long long>(lane) * step;
+        const unsigned le =
+            __ballot_sync(0xffffffffu, lane == 0 || (at < hi && __ldg(rpt + at) <= e));
+        // the true lanes are a prefix for a valid row pointer
+        const int last = 31 - __clz(le);
+        lo += last * step;
+        hi = min(hi, lo + step);
+    }
+    return lo;
+}
+
+template<typename V>
+__global__ __launch_bounds__(256) void k_tr_scatter(const int32_t* __restrict__ a_rpt,
+                                                    const int32_t* __restrict__ a_col,
+                                                    const V* __restrict__ a_val, int32_t m,
+                                                    int32_t nnz,
+                                                    const int32_t* __restrict__ t_rpt,
+                                                    const int32_t* __restrict__ rank,
+                                                    TrRec* __restrict__ recs) {
+    const int lane = threadIdx.x & 31;
+    const long long tile = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) +
+                           (threadIdx.x >> 5);
+    const long long e0 = tile * kScatterTile;
+    if (e0 >= nnz) return;  // uniform over the warp
+    const int e1 = static_cast<int>(min(e0 + kScatterTile, static_cast<long long>(nnz))) - 1;
+    const int rlo = warp_row_of(a_rpt, m, static_cast<int>(e0));
+    const int rhi = warp_row_of(a_rpt, m, e1);
+    int pos[kScatterPer];
+#pragma unroll
+    for (int k = 0; k < kScatterPer; k++) {
+        const long long e = e0 + k * kWarp + lane;
+        pos[k] = -1;
+        if (e <= e1) {
+            const int r = __ldg(rank + e);
+            if (r >= 0) pos[k] = __ldg(t_rpt + __ldg(a_col + e)) + r;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kScatterPer; k++) {
+        const int e = static_cast<int>(e0 + k * kWarp + lane);
+        if (pos[k] < 0) continue;
+        int lo = rlo;
+        for (int len = rhi - rlo + 1; len > 1;) {
+            const int half = len >> 1;
+            lo = __ldg(a_rpt + lo + half) <= e ? lo + half : lo;
+            len -= half;
+        }
+        recs[pos[k]] = TrRec{(static_cast<uint64_t>(static_cast<uint32_t>(lo)) << 32) |
+                                 static_cast<uint32_t>(e),
+                             val_bits<V>(__ldg(a_val + e))};
+    }
+}
+
+// ---- 4. the rows' records in key order ---------------------------------------
+// Rows of up to kTrFlat records: a warp takes rows_per_warp consecutive rows of
+// T and walks their records flat, a lane per record; the record's place in its
+// row is the number of smaller keys there (one broadcast read per record of
+// the row, most from L1: cheaper than a warp's sorting network for the short
+// rows of a graph and free of its 64-bit shuffles).  It runs over all rows and
+// leaves the longer ones to their bins' kernels.
+constexpr int kTrFlat = 128;
+
+template<typename V>
+__global__ __launch_bounds__(256) void k_tr_place(const int32_t* __restrict__ t_rpt, int32_t n,
+                                                  int32_t rows_per_warp,
+                                                  const TrRec* __restrict__ recs,
+                                                  int32_t* __restrict__ t_col,
+                                                  V* __restrict__ t_val) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const long long r0 = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) +
+                          (threadIdx.x >> 5)) * rows_per_warp;
+    if (r0 >= n) return;  // uniform over the warp
+    int t0 = 0;
+    int len = 0;
+    if (lane < rows_per_warp && r0 + lane < n) {
+        t0 = __ldg(t_rpt + r0 + lane);
+        len = __ldg(t_rpt + r0 + lane + 1) - t0;
+        if (len > kTrFlat) len = 0;
+    }
+    const int inc = team_inclusive_scan<kWarp>(kFull, len, lane);
+    const int total = __shfl_sync(kFull, inc, 31);
+    for (int f0 = 0; f0 < total; f0 += kWarp) {  // uniform over the warp
+        const int f = f0 + lane;
+        // record f's row: the first lane with inc > f
+        int j = -1;
+#pragma unroll
+        for (int step = 16; step >= 1; step >>= 1) {
+            const int v = __shfl_sync(kFull, inc, (j + step) & 31);
+            if (v <= f) j += step;
+        }
+        j = (j + 1) & 31;
+        const int start = __shfl_sync(kFull, t0, j);
+        const int before = __shfl_sync(kFull, inc - len, j);
+        const int count = __shfl_sync(kFull, len, j);
+        if (f < total) {
+            const TrRec mine = recs[start + (f - before)];
+            int place = 0;
+#pragma unroll 4
+            for (int i = 0; i < count; i++) place += __ldg(&recs[start + i].key) < mine.key;
+            t_col[start + place] = static_cast<int32_t>(mine.key >> 32);
+            t_val[start + place] = val_of<V>(mine.val);
+        }
+    }
+}
+
 template<typename V>
 __device__ __forceinline__ void store_entry(const ProductArgs& p, int32_t at, uint64_t key) {
     p.c_col[at] = static_cast<int32_t>(key >> 32);
     static_cast<V*>(p.c_val)[at] =
         __ldg(static_cast<const V*>(p.a_val) + static_cast<uint32_t>(key & 0xffffffffu));
-}
-
-// ---- 1. column counts -------------------------------------------------------
-// A column index outside [0, n) is not counted; the host sees the total fall
-// short of nnz and reports the operand as invalid.
-__global__ __launch_bounds__(256) void k_col_count(const int32_t* __restrict__ col, int32_t nnz,
-                                                   int32_t n, int32_t* __restrict__ cnt) {
-    const int lane = threadIdx.x & 31;
-    const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-    // the loop bound is warp-uniform, so every lane joins each match
-    for (long long base = static_cast<long long>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31);
-         base < nnz; base += stride) {
-        const long long e = base + lane;
-        int32_t c = e < nnz ? __ldg(col + e) : -1;
-        if (c >= n) c = -1;
-        const unsigned peers = __match_any_sync(0xffffffffu, c);
-        if (c >= 0 && lane == __ffs(peers) - 1) atomicAdd(cnt + c, __popc(peers));
-    }
-}
-
-// ---- 3. scatter of keys -----------------------------------------------------
-// One warp per row of A; lanes over the row's entries.  Entries whose column
-// is outside [0, n) were not counted and are skipped.
-__global__ __launch_bounds__(256) void k_tr_scatter(const int32_t* __restrict__ a_rpt,
-                                                    const int32_t* __restrict__ a_col, int32_t m,
-                                                    int32_t n, const int32_t* __restrict__ t_rpt,
-                                                    int32_t* __restrict__ cursor,
-                                                    uint64_t* __restrict__ keys) {
-    const int lane = threadIdx.x & 31;
-    const int warps = gridDim.x * (blockDim.x >> 5);
-    for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < m; r += warps) {
-        const int s0 = __ldg(a_rpt + r);
-        const int s1 = __ldg(a_rpt + r + 1);
-        for (int e = s0 + lane; e < s1; e += 32) {
-            const int c = __ldg(a_col + e);
-            if (c < 0 || c >= n) continue;
-            const int pos = __ldg(t_rpt + c) + atomicAdd(cursor + c, 1);
-            keys[pos] = (static_cast<uint64_t>(static_cast<uint32_t>(r)) << 32) |
-                        static_cast<uint32_t>(e);
-        }
-    }
-}
-
-// ---- 4. per-bin row sorts ---------------------------------------------------
-// Rows of up to 32 keys: one warp per row, the network in registers.
-template<typename V, int THREADS>
-__global__ __launch_bounds__(THREADS) void k_tr_sort_warp(ProductArgs p) {
-    const int lane = threadIdx.x & 31;
-    const int rid = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5);
-    if (rid >= p.nrows) return;  // warp-uniform
-    const int row = p.rows[rid];
-    const int t0 = p.c_rpt[row];
-    const int len = p.c_rpt[row + 1] - t0;
-    uint64_t v = lane < len ? p.keys[t0 + lane] : kKeyInf;
-#pragma unroll
-    for (int k = 2; k <= 32; k <<= 1) {
-        const int half = k >> 1;
-        uint64_t o = __shfl_xor_sync(0xffffffffu, v, k - 1);
-        v = (lane & half) ? (v > o ? v : o) : (v < o ? v : o);
-#pragma unroll
-        for (int j = half >> 1; j > 0; j >>= 1) {
-            o = __shfl_xor_sync(0xffffffffu, v, j);
-            v = (lane & j) ? (v > o ? v : o) : (v < o ? v : o);
-        }
-    }
-    if (lane < len) store_entry<V>(p, t0 + lane, v);
 }
 
 // Rows of up to CAP keys: one CTA per row, the keys in shared memory.
@@ -144,13 +275,13 @@ __global__ __launch_bounds__(THREADS) void k_tr_sort_cta(ProductArgs p) {
         if (threadIdx.x == 0) report(p.status, kStCapacity, row, len);
         return;
     }
-    for (int i = threadIdx.x; i < len; i += THREADS) s[i] = p.keys[t0 + i];
+    for (int i = threadIdx.x; i < len; i += THREADS) s[i] = recs_of(p)[t0 + i].key;
     __syncthreads();
     cta_sort_keys<THREADS>(s, len);
     for (int i = threadIdx.x; i < len; i += THREADS) store_entry<V>(p, t0 + i, s[i]);
 }
 
-// Longer rows: one CTA per row, sorting the row's keys in place in global
+// Longer rows: one CTA per row, sorting the row's records in place in global
 // memory (the network's passes stay in L2 for rows of a few MB).
 template<typename V, int THREADS>
 __global__ __launch_bounds__(THREADS) void k_tr_sort_global(ProductArgs p) {
@@ -158,17 +289,30 @@ __global__ __launch_bounds__(THREADS) void k_tr_sort_global(ProductArgs p) {
         const int row = p.rows[rid];
         const int t0 = p.c_rpt[row];
         const int len = p.c_rpt[row + 1] - t0;
-        uint64_t* a = p.keys + t0;
+        TrRec* a = reinterpret_cast<TrRec*>(p.keys) + t0;
         cta_sort_keys<THREADS>(a, len);
-        for (int i = threadIdx.x; i < len; i += THREADS) store_entry<V>(p, t0 + i, a[i]);
+        for (int i = threadIdx.x; i < len; i += THREADS) {
+            p.c_col[t0 + i] = static_cast<int32_t>(a[i].key >> 32);
+            static_cast<V*>(p.c_val)[t0 + i] = val_of<V>(a[i].val);
+        }
         __syncthreads();
     }
 }
 
-template<typename V, int THREADS>
-cudaError_t launch_warp(const ProductArgs& p, cudaStream_t s) {
-    constexpr int R = THREADS / 32;
-    k_tr_sort_warp<V, THREADS><<<(p.nrows + R - 1) / R, THREADS, 0, s>>>(p);
+// Rows per warp of k_tr_place for about kPlaceEntries records a warp.
+constexpr int64_t kPlaceEntries = 256;
+
+// Every row of T, not only this bin's list: the list would cost a gather per
+// row, and the rows of other bins only a row-pointer read.
+template<typename V>
+cudaError_t launch_place(const ProductArgs& p, cudaStream_t s) {
+    const int32_t n = p.n_cols;  // rows of T
+    const int64_t nnz = p.words; // entries of T
+    int rows = 1;
+    while (rows < kWarp && (2 * rows) * nnz <= kPlaceEntries * n) rows *= 2;
+    const int64_t warps = (static_cast<int64_t>(n) + rows - 1) / rows;
+    k_tr_place<V><<<static_cast<unsigned>((warps + 7) / 8), 256, 0, s>>>(
+        p.c_rpt, n, rows, recs_of(p), p.c_col, static_cast<V*>(p.c_val));
     return cudaGetLastError();
 }
 
@@ -192,7 +336,7 @@ struct TransposeLadder {
 
 template<typename V>
 const BinLauncher TransposeLadder<V>::bins[4] = {
-    {BinKind::Team, 32, 8, 256, 0, "tr_sort_warp32", launch_warp<V, 256>},
+    {BinKind::Team, kTrFlat, 8, 256, 0, "tr_place", launch_place<V>},
     {BinKind::Cta, 2048, 1, 256, sizeof(uint64_t) * 2048, "tr_sort_cta2048",
      launch_cta<V, 256, 2048>},
     {BinKind::Cta, 16384, 1, 1024, sizeof(uint64_t) * 16384, "tr_sort_cta16384",
@@ -227,21 +371,27 @@ cudaError_t transpose_prepare() {
 }
 
 cudaError_t launch_col_count(const int32_t* col, int32_t nnz, int32_t n, int32_t* cnt,
-                             cudaStream_t s) {
+                             int32_t* rank, cudaStream_t s) {
     if (nnz <= 0) return cudaSuccess;
-    long long g = (static_cast<long long>(nnz) + 255) / 256;
+    long long g = (static_cast<long long>(nnz) + 256 * kCountUnroll - 1) / (256 * kCountUnroll);
     if (g > 148 * 16) g = 148 * 16;
-    k_col_count<<<static_cast<int>(g), 256, 0, s>>>(col, nnz, n, cnt);
+    k_col_count<<<static_cast<int>(g), 256, 0, s>>>(col, nnz, n, cnt, rank);
     return cudaGetLastError();
 }
 
-cudaError_t launch_tr_scatter(const int32_t* a_rpt, const int32_t* a_col, int32_t m, int32_t n,
-                              const int32_t* t_rpt, int32_t* cursor, uint64_t* keys,
-                              cudaStream_t s) {
-    if (m <= 0) return cudaSuccess;
-    long long g = (static_cast<long long>(m) + 7) / 8;
-    if (g > 148 * 16) g = 148 * 16;
-    k_tr_scatter<<<static_cast<int>(g), 256, 0, s>>>(a_rpt, a_col, m, n, t_rpt, cursor, keys);
+cudaError_t launch_tr_scatter(const int32_t* a_rpt, const int32_t* a_col, const void* a_val,
+                              int value_bytes, int32_t m, int32_t nnz, const int32_t* t_rpt,
+                              const int32_t* rank, uint64_t* recs, cudaStream_t s) {
+    if (m <= 0 || nnz <= 0) return cudaSuccess;
+    constexpr int kPerCta = 8 * kScatterTile;
+    const unsigned g = static_cast<unsigned>((static_cast<long long>(nnz) + kPerCta - 1) / kPerCta);
+    TrRec* out = reinterpret_cast<TrRec*>(recs);
+    if (value_bytes == 8)
+        k_tr_scatter<double><<<g, 256, 0, s>>>(a_rpt, a_col, static_cast<const double*>(a_val), m,
+                                               nnz, t_rpt, rank, out);
+    else
+        k_tr_scatter<float><<<g, 256, 0, s>>>(a_rpt, a_col, static_cast<const float*>(a_val), m,
+                                              nnz, t_rpt, rank, out);
     return cudaGetLastError();
 }
 

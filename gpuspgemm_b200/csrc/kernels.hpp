@@ -55,7 +55,8 @@ struct ProductArgs {
     int32_t cluster;        // CTAs per cluster
     int32_t* fail_rows;     // rows that spilled out of a cluster table
     int32_t* fail_count;
-    // transpose: per entry of T, (row of A << 32 | position in A)
+    // transpose: a 16-byte record per entry of T, its first word (row of A << 32
+    // | position in A); n_cols and words are then T's rows and entries
     uint64_t* keys;
     // one-pass fill: c_rpt gives each row a slot of its NIP entries (an upper
     // bound); the kernel writes the row's exact nnz here (nullptr: c_rpt is
@@ -233,15 +234,17 @@ cudaError_t launch_unpack(const int32_t* c_rpt, int32_t* c_col, const int32_t* r
                           int32_t count, int32_t rows, int32_t nnz, int32_t* rpt_out,
                           int32_t* pos_out, cudaStream_t s);
 // CSR transpose (k_transpose.cu): row-sort ladder (key = length of a row of
-// A^T), column counts, and the keyed scatter.
+// A^T), column counts with each entry's rank in its column, and the scatter.
 int transpose_ladder_f64(const BinLauncher** out);
 int transpose_ladder_f32(const BinLauncher** out);
 cudaError_t transpose_prepare();
 cudaError_t launch_col_count(const int32_t* col, int32_t nnz, int32_t n, int32_t* cnt,
-                             cudaStream_t s);
-cudaError_t launch_tr_scatter(const int32_t* a_rpt, const int32_t* a_col, int32_t m, int32_t n,
-                              const int32_t* t_rpt, int32_t* cursor, uint64_t* keys,
-                              cudaStream_t s);
+                             int32_t* rank, cudaStream_t s);
+// recs: kTrRecBytes per entry of A
+constexpr size_t kTrRecBytes = 16;
+cudaError_t launch_tr_scatter(const int32_t* a_rpt, const int32_t* a_col, const void* a_val,
+                              int value_bytes, int32_t m, int32_t nnz, const int32_t* t_rpt,
+                              const int32_t* rank, uint64_t* recs, cudaStream_t s);
 // NIP of many independent pairs in one launch (spgemm_get_nip_many).
 struct NipPair {
     const int32_t* a_col;   // A_i's column indices (nnz entries)

@@ -1565,9 +1565,9 @@ spgemm_status product_host(spgemm_handle_s* h, const spgemm_csr_view* A,
 }
 
 // ---- CSR transpose -----------------------------------------------------------
-// T = A^T with sorted columns (k_transpose.cu): column counts, the binning pass
-// with the scan (T.rpt and length bins of T's rows), a keyed scatter, then one
-// sort kernel per non-empty length bin.  One host synchronisation (the bin
+// T = A^T with sorted columns (k_transpose.cu): column counts and ranks, the
+// binning pass with the scan (T.rpt and length bins of T's rows), a scatter of
+// records, then one ordering kernel per non-empty length bin.  One host synchronisation (the bin
 // sizes), like each binning pass of a product.
 template<typename V>
 spgemm_status transpose(spgemm_handle_s* h, const spgemm_csr_view* A, spgemm_csr_out* T,
@@ -1591,12 +1591,10 @@ spgemm_status transpose(spgemm_handle_s* h, const spgemm_csr_view* A, spgemm_csr
     B200_TRY(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&T->rpt),
                                      sizeof(int32_t) * (size_t(n) + 1), h->pool, stream));
     uint64_t* keys = nullptr;
-    int32_t* cursor = nullptr;
     auto bail = [&](spgemm_status st) {
         const std::string msg = g_last_error;
         cudaStreamSynchronize(stream);
         if (keys) cudaFreeAsync(keys, stream);
-        if (cursor) cudaFreeAsync(cursor, stream);
         spgemm_csr_free(T, stream);
         cudaStreamSynchronize(stream);
         h->prof.clear();
@@ -1632,8 +1630,12 @@ spgemm_status transpose(spgemm_handle_s* h, const spgemm_csr_view* A, spgemm_csr
         B200_CUDA(cudaStreamSynchronize(stream), "synchronize");
         return SPGEMM_OK;
     }
+    // T.col holds the entries' ranks until the last step writes it
+    B200_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&T->col),
+                                      sizeof(int32_t) * size_t(nnz) + 16, h->pool, stream),
+              "allocate T.col");
     B200_STEP(timed(h, "col_count", 1, -1, nnz, stream, [&](cudaStream_t ss) {
-        return launch_col_count(A->col, nnz, n, T->rpt, ss);
+        return launch_col_count(A->col, nnz, n, T->rpt, T->col, ss);
     }));
     const Ladder lad = make_ladder(tl, ntl, h->min_tr_bin);
     const int nctas = bin_ctas(n);
@@ -1648,18 +1650,12 @@ spgemm_status transpose(spgemm_handle_s* h, const spgemm_csr_view* A, spgemm_csr
                                   ss);
     }));
     B200_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&keys),
-                                      sizeof(uint64_t) * size_t(nnz), h->pool, stream),
-              "allocate transpose keys");
-    B200_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&cursor),
-                                      sizeof(int32_t) * size_t(n), h->pool, stream),
-              "allocate transpose cursors");
-    B200_CUDA(cudaMemsetAsync(cursor, 0, sizeof(int32_t) * size_t(n), stream), "memset cursors");
+                                      kTrRecBytes * size_t(nnz), h->pool, stream),
+              "allocate transpose records");
     B200_STEP(timed(h, "tr_scatter", 3, -1, m, stream, [&](cudaStream_t ss) {
-        return launch_tr_scatter(A->rpt, A->col, m, n, T->rpt, cursor, keys, ss);
+        return launch_tr_scatter(A->rpt, A->col, A->val, static_cast<int>(sizeof(V)), m, nnz,
+                                 T->rpt, T->col, keys, ss);
     }));
-    B200_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&T->col),
-                                      sizeof(int32_t) * size_t(nnz) + 16, h->pool, stream),
-              "allocate T.col");
     B200_CUDA(cudaMallocFromPoolAsync(&T->val, sizeof(V) * size_t(nnz), h->pool, stream),
               "allocate T.val");
     T->nnz = nnz;
@@ -1678,11 +1674,11 @@ spgemm_status transpose(spgemm_handle_s* h, const spgemm_csr_view* A, spgemm_csr
     pa.c_val = T->val;
     pa.status = s.status;
     pa.keys = keys;
+    pa.n_cols = n;
+    pa.words = nnz;
     B200_STEP(launch_bins(h, tl, ntl, 4, plan, s.bins2, pa, stream));
-    B200_CUDA(cudaFreeAsync(keys, stream), "free transpose keys");
+    B200_CUDA(cudaFreeAsync(keys, stream), "free transpose records");
     keys = nullptr;
-    B200_CUDA(cudaFreeAsync(cursor, stream), "free transpose cursors");
-    cursor = nullptr;
     B200_CUDA(cudaMemcpyAsync(&h->mirror->status, s.status, sizeof(DevStatus),
                               cudaMemcpyDeviceToHost, stream),
               "read status");
