@@ -9,6 +9,12 @@
 //   scatter  stable scatter of row ids (+ the exclusive scan into C.rpt)
 // The scatter is stable: rows of a bin keep ascending row order, so the bin
 // kernels read A and write C in order.
+//
+// Up to kAppendMaxRows rows a pass is ONE kernel instead: every bin has a row
+// list of its own (room for all rows), and a CTA reserves its rows' places with
+// one atomic per bin, so no CTA needs another's histogram.  Rows are ascending
+// within a CTA's share of a list and the shares come in about the CTAs' order,
+// which is all the bin kernels' locality needs.
 #include "cta.cuh"
 #include "kernels.hpp"
 
@@ -145,6 +151,260 @@ __global__ __launch_bounds__(kNipThreads) void k_nip_hist(
     }
 }
 
+// ---- append binning: one launch a pass ---------------------------------------
+// The row lists: bin b's rows at lists[b * stride ...], their number in
+// plan->bin_size[b] (zeroed before the pass).  A CTA counts its rows per bin in
+// shared memory, reserves its share of every list with one global atomic per
+// bin and writes the rows there.  (Three kernels with a one-CTA scan between
+// them took 33 us on a small product and 51 us on 1M rows; one takes 9 and the
+// NIP pass's own time.)
+struct AppendShared {
+    int32_t next[kMaxBins];  // per bin: the CTA's count, then its next free place
+};
+
+// Before the first append_count: clear (a barrier must follow).
+__device__ __forceinline__ void append_clear(AppendShared& sh) {
+    if (threadIdx.x < kMaxBins) sh.next[threadIdx.x] = 0;
+}
+
+// Count a warp's 32 rows (bin < 0: in no list).
+__device__ __forceinline__ void append_count(AppendShared& sh, int bin) {
+    const unsigned peers = __match_any_sync(0xffffffffu, bin);
+    if (bin >= 0 && (threadIdx.x & 31) == static_cast<unsigned>(__ffs(peers) - 1))
+        atomicAdd(&sh.next[bin], __popc(peers));
+}
+
+// After a barrier: turn the counts into places (a barrier must follow).
+__device__ __forceinline__ void append_reserve(AppendShared& sh, Plan* plan) {
+    if (threadIdx.x < kMaxBins) {
+        const int c = sh.next[threadIdx.x];
+        sh.next[threadIdx.x] = c > 0 ? atomicAdd(&plan->bin_size[threadIdx.x], c) : 0;
+    }
+}
+
+// Write a warp's 32 rows, in the order of the append_count calls.
+__device__ __forceinline__ void append_rows(AppendShared& sh, int bin, int32_t row,
+                                            int32_t* __restrict__ lists, int64_t stride) {
+    const int lane = threadIdx.x & 31;
+    const unsigned peers = __match_any_sync(0xffffffffu, bin);
+    const int leader = __ffs(peers) - 1;
+    int at = 0;
+    if (bin >= 0 && lane == leader) at = atomicAdd(&sh.next[bin], __popc(peers));
+    at = __shfl_sync(0xffffffffu, at, leader);
+    if (bin >= 0) lists[bin * stride + at + __popc(peers & ((1u << lane) - 1u))] = row;
+}
+
+// Per-row keys of the CTA's rows -- warp w's group j holds rows
+// (w * PER + j) * 32 + lane of the CTA -- into the lists, the plan's total and
+// max, and, when `off` is given, each row's slot start: the CTA's slots follow
+// one another from a base taken with one atomic on the total (so slots are in
+// row order only within a CTA's rows; a row's slot holds its key's entries).
+template<int PER>
+__device__ __forceinline__ void append_keys(const int32_t (&key)[PER], long long tot, int32_t row0,
+                                            int32_t m, int32_t* __restrict__ off,
+                                            int32_t* __restrict__ lists, int64_t stride,
+                                            Plan* __restrict__ plan, const Ladder& lad) {
+    constexpr int NW = kBinThreads / kWarp;
+    __shared__ AppendShared sh;
+    __shared__ long long s_sum[NW];
+    __shared__ int32_t s_max[NW];
+    __shared__ long long s_base;
+    const int lane = threadIdx.x & 31;
+    const int w = threadIdx.x >> 5;
+    int32_t mx = 0;
+    append_clear(sh);
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        mx = max(mx, key[j]);
+        append_count(sh, key[j] > 0 ? find_bin(lad, key[j]) : -1);
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    tot = warp_sum_ll(tot);
+    if (lane == 0) {
+        s_sum[w] = tot;
+        s_max[w] = mx;
+    }
+    __syncthreads();
+    append_reserve(sh, plan);
+    if (threadIdx.x == kMaxBins) {
+        long long t = 0;
+        int32_t cmx = 0;
+        for (int i = 0; i < NW; i++) {
+            const long long x = s_sum[i];
+            s_sum[i] = t;
+            t += x;
+            cmx = max(cmx, s_max[i]);
+        }
+        s_base = t == 0 ? 0
+                        : static_cast<long long>(
+                              atomicAdd(reinterpret_cast<unsigned long long*>(&plan->total_key),
+                                        static_cast<unsigned long long>(t)));
+        if (cmx > 0) atomicMax(&plan->max_key, cmx);
+    }
+    __syncthreads();
+    // int arithmetic: it wraps only when the total leaves int32, and then the
+    // slots are not used (two passes)
+    int run = static_cast<int>(s_base + s_sum[w]);
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int32_t r = row0 + (w * PER + j) * kWarp + lane;
+        append_rows(sh, key[j] > 0 ? find_bin(lad, key[j]) : -1, r, lists, stride);
+        if (off != nullptr) {
+            const int inc = team_inclusive_scan<kWarp>(0xffffffffu, key[j], lane);
+            if (r < m) off[r] = run + inc - key[j];
+            run += __shfl_sync(0xffffffffu, inc, kWarp - 1);
+        }
+    }
+}
+
+// NIP of the warp's 32 rows [s0, s1) of A entries, a row per lane.  Rows of up
+// to 31 entries take a lane each; rows of up to kNipMedium entries eight lanes,
+// four rows at a time; longer ones the warp, one after another.  (Bound by the
+// latency of a_col -> b_rpt gathers: the medium class keeps four rows' gathers
+// in flight where the warp-per-row walk had one -- 35,937 rows of 84 entries
+// 0.170 -> 0.02 ms, with 256 rows a CTA instead of 1,024.)
+constexpr int kNipMedium = 128;
+
+__device__ __forceinline__ long long nip_of_rows(const int32_t* __restrict__ a_col,
+                                                 const int32_t* __restrict__ b_rpt, int s0,
+                                                 int s1) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int len = s1 - s0;
+    long long nip = 0;
+    if (len < kWarp) {
+#pragma unroll 4
+        for (int p = s0; p < s1; p++) {
+            const int c = __ldg(a_col + p);
+            nip += __ldg(b_rpt + c + 1) - __ldg(b_rpt + c);
+        }
+    }
+    for (unsigned mid = __ballot_sync(kFull, len >= kWarp && len <= kNipMedium); mid != 0u;) {
+        // the next four medium rows, one per eight lanes
+        int pick = -1;
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            if (mid == 0u) break;  // uniform over the warp
+            const int i = __ffs(mid) - 1;
+            mid &= mid - 1u;
+            if ((lane >> 3) == t) pick = i;
+        }
+        const int rs = __shfl_sync(kFull, s0, pick & 31);
+        const int re = __shfl_sync(kFull, s1, pick & 31);
+        constexpr int U = 4;
+        long long part = 0;
+        if (pick >= 0) {
+            for (int p0 = rs + (lane & 7); p0 < re; p0 += U * 8) {
+                int c[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) c[u] = p0 + u * 8 < re ? __ldg(a_col + p0 + u * 8) : -1;
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    if (c[u] >= 0) part += __ldg(b_rpt + c[u] + 1) - __ldg(b_rpt + c[u]);
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) part += __shfl_xor_sync(kFull, part, o);
+        // hand each row's sum to the lane that holds the row
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            const int to = __shfl_sync(kFull, pick, t * 8);
+            const long long sum = __shfl_sync(kFull, part, t * 8);
+            if (lane == to) nip = sum;
+        }
+    }
+    for (unsigned longm = __ballot_sync(kFull, len > kNipMedium); longm != 0u;
+         longm &= longm - 1u) {
+        const int i = __ffs(longm) - 1;
+        const int rs = __shfl_sync(kFull, s0, i);
+        const int re = __shfl_sync(kFull, s1, i);
+        constexpr int U = 8;
+        long long part = 0;
+        for (int p0 = rs + lane; p0 < re; p0 += U * kWarp) {
+            int c[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int p = p0 + u * kWarp;
+                c[u] = p < re ? __ldg(a_col + p) : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (c[u] >= 0) part += __ldg(b_rpt + c[u] + 1) - __ldg(b_rpt + c[u]);
+        }
+        part = warp_sum_ll(part);
+        if (lane == i) nip = part;
+    }
+    return nip;
+}
+
+// Rows per CTA: kBinRowsPerCta from kAppendWide rows on, where that fills the
+// chip (148 SMs x 4 CTAs) and shares the reservations; 256 below.
+constexpr int kAppendPer = kBinRowsPerCta / kBinThreads;
+constexpr int32_t kAppendWide = 148 * 4 * kBinRowsPerCta;
+
+template<int PER>
+__global__ __launch_bounds__(kBinThreads) void k_nip_append(
+    const int32_t* __restrict__ a_rpt, const int32_t* __restrict__ a_col,
+    const int32_t* __restrict__ b_rpt, int32_t m, int32_t* __restrict__ c_rpt,
+    int32_t* __restrict__ off, int32_t* __restrict__ lists, int64_t stride,
+    Plan* __restrict__ plan, DevStatus* __restrict__ st, const __grid_constant__ Ladder lad) {
+    const int lane = threadIdx.x & 31;
+    const int w = threadIdx.x >> 5;
+    const int32_t row0 = blockIdx.x * (PER * kBinThreads);
+    int32_t key[PER];
+    long long tot = 0;
+#pragma unroll 1
+    for (int j = 0; j < PER; j++) {
+        const int32_t r = row0 + (w * PER + j) * kWarp + lane;
+        int s0 = 0;
+        int s1 = 0;
+        if (r < m) {
+            s0 = a_rpt[r];
+            s1 = a_rpt[r + 1];
+        }
+        const long long nip = nip_of_rows(a_col, b_rpt, s0, s1);
+        int32_t k = 0;
+        if (r < m) {
+            if (nip > INT32_MAX) {
+                report(st, kStNipOverflow, r);
+                k = INT32_MAX;
+            } else {
+                k = static_cast<int32_t>(nip);
+            }
+            c_rpt[r] = k;
+            tot += nip;
+        }
+#pragma unroll
+        for (int q = 0; q < PER; q++)
+            if (q == j) key[q] = k;
+    }
+    append_keys<PER>(key, tot, row0, m, off, lists, stride, plan, lad);
+}
+
+// The same from keys in memory (a NIP per row that an earlier pass wrote).
+template<int PER>
+__global__ __launch_bounds__(kBinThreads) void k_key_append(const int32_t* __restrict__ keys,
+                                                            int32_t m, int32_t* __restrict__ off,
+                                                            int32_t* __restrict__ lists,
+                                                            int64_t stride,
+                                                            Plan* __restrict__ plan,
+                                                            const __grid_constant__ Ladder lad) {
+    const int lane = threadIdx.x & 31;
+    const int w = threadIdx.x >> 5;
+    const int32_t row0 = blockIdx.x * (PER * kBinThreads);
+    int32_t key[PER];
+    long long tot = 0;
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int32_t r = row0 + (w * PER + j) * kWarp + lane;
+        key[j] = r < m ? keys[r] : 0;
+        tot += key[j];
+    }
+    append_keys<PER>(key, tot, row0, m, off, lists, stride, plan, lad);
+}
+
 // ---- pass 1': nnz histogram + per-CTA nnz sums ----------------------------
 __global__ __launch_bounds__(kBinThreads) void k_nnz_hist(
     const int32_t* __restrict__ c_rpt, int32_t m, int32_t* __restrict__ hist,
@@ -271,13 +531,9 @@ __device__ __forceinline__ int offmap_pad(int j) { return j + (j >> 5); }
 __global__ __launch_bounds__(kOffMapThreads) void k_bin_offsets_map(
     const int32_t* __restrict__ src_hist, int32_t* __restrict__ hist, int32_t nctas,
     const __grid_constant__ Ladder src, int64_t* __restrict__ cta_sum, Plan* __restrict__ plan,
-    const __grid_constant__ Ladder lad, const Ladder* __restrict__ dlad,
-    unsigned long long* __restrict__ zero, int32_t nzero) {
+    const __grid_constant__ Ladder lad, const Ladder* __restrict__ dlad) {
     constexpr int NW = kOffMapThreads / kWarp;
     constexpr int PADDED = kOffMapChunk + kOffMapChunk / kWarp;
-    // words a later kernel of the product needs zeroed (the row pointer's
-    // look-back state): cleared here instead of by a memset of their own
-    for (int i = threadIdx.x; i < nzero; i += kOffMapThreads) zero[i] = 0ull;
     static_assert(NW > kMaxBins, "a warp per bin and one for the CTA sums");
     static_assert(kBinRowsPerCta < 65536, "16-bit counts");
     __shared__ uint16_t s_cnt[kMaxBins][PADDED + 1];
@@ -460,11 +716,10 @@ __global__ __launch_bounds__(kBinThreads) void k_bin_scatter(
 // a CTA): 8 bytes of traffic per row, where a one-bin pass of the binning
 // kernels takes three launches and also writes a row list.
 constexpr int kScanThreads = 256;
-constexpr int kScanPer = kScanTile / kScanThreads;  // rows per thread
-static_assert(kScanPer * kScanThreads == kScanTile, "tile");
+static_assert(kScanTile % kScanThreads == 0 && kScanAppendTile % kScanThreads == 0, "tile");
 
 // the tile in shared memory, one padding word per 32 (thread t reads its
-// kScanPer consecutive rows without bank conflicts)
+// consecutive rows without bank conflicts)
 __device__ __forceinline__ int scan_pad(int i) { return i + (i >> 5); }
 
 // One launch, the tiles chained by decoupled look-back.
@@ -484,21 +739,28 @@ constexpr unsigned long long kTilePrefix = 2ull << 62;
 constexpr unsigned long long kTileValue = (1ull << 62) - 1ull;
 constexpr int kLookbackSpins = 1 << 20;
 
-__global__ __launch_bounds__(kScanThreads) void k_rpt_scan1(int32_t* __restrict__ cnt, int32_t m,
-                                                            int32_t ntiles,
-                                                            unsigned long long* __restrict__ state,
-                                                            Plan* __restrict__ plan,
-                                                            DevStatus* __restrict__ st) {
-    constexpr int NW = kScanThreads / kWarp;
+// With APPEND the tile's rows also join their bins' lists (the two-pass scan
+// pass and the transpose's: row pointer and bins in one launch).  The tile is
+// then kScanAppendTile rows: binning walks a thread's rows one after another,
+// and 16 of them took 20 us on a small product, where 4 take 9.
+template<bool APPEND, int TILE>
+__device__ __forceinline__ void scan1_tile(int32_t* __restrict__ cnt, int32_t m, int32_t ntiles,
+                                           unsigned long long* __restrict__ state,
+                                           Plan* __restrict__ plan, DevStatus* __restrict__ st,
+                                           int32_t* __restrict__ lists, int64_t stride,
+                                           const Ladder& lad) {    constexpr int NW = kScanThreads / kWarp;
+    constexpr int PER = TILE / kScanThreads;  // rows per thread
     constexpr unsigned kAll = 0xffffffffu;
-    __shared__ int32_t s_row[kScanTile + kScanTile / 32];
+    __shared__ int32_t s_row[TILE + TILE / 32];
     __shared__ int32_t s_wtot[NW];
     __shared__ int32_t s_wmax[NW];
     __shared__ int32_t s_tile;
     __shared__ long long s_base;
+    __shared__ AppendShared s_app;
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int w = tid >> 5;
+    if constexpr (APPEND) append_clear(s_app);
     if (tid == 0) s_tile = static_cast<int32_t>(atomicAdd(state, 1ull));
     __syncthreads();
     const int tile = s_tile;
@@ -506,20 +768,23 @@ __global__ __launch_bounds__(kScanThreads) void k_rpt_scan1(int32_t* __restrict_
         if (tid == 0) report(st, kStIndex, tile, ntiles);
         return;
     }
-    const long long r0 = static_cast<long long>(tile) * kScanTile;
+    const long long r0 = static_cast<long long>(tile) * TILE;
 #pragma unroll
-    for (int k = 0; k < kScanPer; k++) {
+    for (int k = 0; k < PER; k++) {
         const int j = k * kScanThreads + tid;
-        s_row[scan_pad(j)] = r0 + j < m ? cnt[r0 + j] : 0;
+        const int32_t c = r0 + j < m ? cnt[r0 + j] : 0;
+        s_row[scan_pad(j)] = c;
+        if constexpr (APPEND) append_count(s_app, c > 0 ? find_bin(lad, c) : -1);
     }
     __syncthreads();
-    // thread tid: rows [tid * kScanPer, (tid + 1) * kScanPer) of the tile
-    int v[kScanPer];
+    if constexpr (APPEND) append_reserve(s_app, plan);
+    // thread tid: rows [tid * PER, (tid + 1) * PER) of the tile
+    int v[PER];
     int run = 0;
     int mx = 0;
 #pragma unroll
-    for (int k = 0; k < kScanPer; k++) {
-        v[k] = s_row[scan_pad(tid * kScanPer + k)];
+    for (int k = 0; k < PER; k++) {
+        v[k] = s_row[scan_pad(tid * PER + k)];
         run += v[k];
         mx = max(mx, v[k]);
     }
@@ -569,19 +834,28 @@ __global__ __launch_bounds__(kScanThreads) void k_rpt_scan1(int32_t* __restrict_
             s_base = excl;
         }
     }
+    if constexpr (APPEND) {
+        // (the places were reserved before the scan's barriers)
+        for (int k = 0; k < PER; k++) {
+            const int j = k * kScanThreads + tid;
+            const int32_t c = s_row[scan_pad(j)];
+            append_rows(s_app, c > 0 ? find_bin(lad, c) : -1, static_cast<int32_t>(r0 + j), lists,
+                        stride);
+        }
+    }
     __syncthreads();
     const long long base = s_base;
     // int arithmetic inside the tile: it wraps only when the total leaves
     // int32, which the plan's int64 total flags
     int pos = static_cast<int>(base) + inc - run;
 #pragma unroll
-    for (int k = 0; k < kScanPer; k++) {
-        s_row[scan_pad(tid * kScanPer + k)] = pos;
+    for (int k = 0; k < PER; k++) {
+        s_row[scan_pad(tid * PER + k)] = pos;
         pos += v[k];
     }
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < kScanPer; k++) {
+    for (int k = 0; k < PER; k++) {
         const int j = k * kScanThreads + tid;
         if (r0 + j < m) cnt[r0 + j] = s_row[scan_pad(j)];
     }
@@ -591,6 +865,22 @@ __global__ __launch_bounds__(kScanThreads) void k_rpt_scan1(int32_t* __restrict_
         plan->total_key = total;
         plan->overflow = total > INT32_MAX ? 1 : 0;
     }
+}
+
+__global__ __launch_bounds__(kScanThreads) void k_rpt_scan1(int32_t* __restrict__ cnt, int32_t m,
+                                                            int32_t ntiles,
+                                                            unsigned long long* __restrict__ state,
+                                                            Plan* __restrict__ plan,
+                                                            DevStatus* __restrict__ st) {
+    const Ladder none = {};
+    scan1_tile<false, kScanTile>(cnt, m, ntiles, state, plan, st, nullptr, 0, none);
+}
+
+__global__ __launch_bounds__(kScanThreads) void k_rpt_scan_append(
+    int32_t* __restrict__ cnt, int32_t m, int32_t ntiles, unsigned long long* __restrict__ state,
+    Plan* __restrict__ plan, DevStatus* __restrict__ st, int32_t* __restrict__ lists,
+    int64_t stride, const __grid_constant__ Ladder lad) {
+    scan1_tile<true, kScanAppendTile>(cnt, m, ntiles, state, plan, st, lists, stride, lad);
 }
 
 // ---- one-pass fill: compaction of the rows into C ----------------------------
@@ -730,10 +1020,9 @@ cudaError_t launch_nip_hist(const int32_t* a_rpt, const int32_t* a_col, const in
 
 cudaError_t launch_bin_offsets_map(const int32_t* src_hist, int32_t* hist, int32_t nctas,
                                    const Ladder& src, int64_t* cta_sum, Plan* plan,
-                                   const Ladder& lad, const Ladder* dlad, cudaStream_t s,
-                                   unsigned long long* zero, int32_t nzero) {
+                                   const Ladder& lad, const Ladder* dlad, cudaStream_t s) {
     k_bin_offsets_map<<<1, kOffMapThreads, 0, s>>>(src_hist, hist, nctas, src, cta_sum, plan, lad,
-                                                   dlad, zero, nzero);
+                                                   dlad);
     return cudaGetLastError();
 }
 
@@ -742,6 +1031,42 @@ cudaError_t launch_rpt_scan1(int32_t* cnt, int32_t m, unsigned long long* state,
     if (m <= 0) return cudaSuccess;
     const int tiles = rpt_scan_tiles(m);
     k_rpt_scan1<<<tiles, kScanThreads, 0, s>>>(cnt, m, tiles, state, plan, st);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_nip_append(const int32_t* a_rpt, const int32_t* a_col, const int32_t* b_rpt,
+                              int32_t m, int32_t* c_rpt, int32_t* off, int32_t* lists,
+                              int64_t stride, Plan* plan, DevStatus* st, const Ladder& lad,
+                              cudaStream_t s) {
+    if (m <= 0) return cudaSuccess;
+    if (m >= kAppendWide)
+        k_nip_append<kAppendPer><<<(m - 1) / kBinRowsPerCta + 1, kBinThreads, 0, s>>>(
+            a_rpt, a_col, b_rpt, m, c_rpt, off, lists, stride, plan, st, lad);
+    else
+        k_nip_append<1><<<(m - 1) / kBinThreads + 1, kBinThreads, 0, s>>>(
+            a_rpt, a_col, b_rpt, m, c_rpt, off, lists, stride, plan, st, lad);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_key_append(const int32_t* keys, int32_t m, int32_t* off, int32_t* lists,
+                              int64_t stride, Plan* plan, const Ladder& lad, cudaStream_t s) {
+    if (m <= 0) return cudaSuccess;
+    if (m >= kAppendWide)
+        k_key_append<kAppendPer><<<(m - 1) / kBinRowsPerCta + 1, kBinThreads, 0, s>>>(
+            keys, m, off, lists, stride, plan, lad);
+    else
+        k_key_append<1><<<(m - 1) / kBinThreads + 1, kBinThreads, 0, s>>>(keys, m, off, lists,
+                                                                          stride, plan, lad);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_rpt_scan_append(int32_t* cnt, int32_t m, unsigned long long* state, Plan* plan,
+                                   DevStatus* st, int32_t* lists, int64_t stride,
+                                   const Ladder& lad, cudaStream_t s) {
+    if (m <= 0) return cudaSuccess;
+    const int tiles = (m - 1) / kScanAppendTile + 1;
+    k_rpt_scan_append<<<tiles, kScanThreads, 0, s>>>(cnt, m, tiles, state, plan, st, lists, stride,
+                                                     lad);
     return cudaGetLastError();
 }
 

@@ -30,6 +30,11 @@ __device__ __forceinline__ V ldv(const void* base, int i) {
     return __ldg(static_cast<const V*>(base) + i);
 }
 
+// Entries of a row's slot at c0: its exact nnz, or in one-pass mode its NIP.
+__device__ __forceinline__ int slot_entries(const ProductArgs& p, int row, int c0) {
+    return p.row_slot != nullptr ? p.row_slot[row] : p.c_rpt[row + 1] - c0;
+}
+
 // A row of C whose A row holds ONE entry (a_ik at column k) is a_ik times B's
 // row k: its columns are B's (sorted, duplicate-free) and each value is one
 // rounded product, as in Gustavson.  The one-pass fill bins copy such rows
@@ -99,7 +104,7 @@ __global__ __launch_bounds__(THREADS) void k_s2n_team(ProductArgs p) {
     const int row = p.rows[rid];
     const int c0 = p.c_rpt[row];
     // the row's exact nnz, or in one-pass mode its NIP (an upper bound)
-    const int bound = p.c_rpt[row + 1] - c0;
+    const int bound = slot_entries(p, row, c0);
     if (bound > T) {
         if (lane == 0) report(p.status, kStCapacity, row, bound);
         return;
@@ -174,7 +179,7 @@ __global__ __launch_bounds__(THREADS) void k_esc_team(ProductArgs p) {
     int32_t* keys = reinterpret_cast<int32_t*>(smem_raw + L::vals_bytes) + team * T;
     const int row = p.rows[rid];
     const int c0 = p.c_rpt[row];
-    const int nip = p.c_rpt[row + 1] - c0;  // the row's NIP-sized slot
+    const int nip = slot_entries(p, row, c0);
     if (nip > NMAX || p.row_nnz == nullptr) {
         if (lane == 0) report(p.status, kStCapacity, row, nip);
         return;
@@ -291,7 +296,7 @@ __global__ __launch_bounds__(THREADS) void k_esc_warp(ProductArgs p) {
     if (lane < nr) {
         row = p.rows[r0 + lane];
         c0 = p.c_rpt[row];
-        nip = p.c_rpt[row + 1] - c0;  // the row's NIP-sized slot
+        nip = slot_entries(p, row, c0);
         a0 = p.a_rpt[row];
         deg = p.a_rpt[row + 1] - a0;
         if (nip > CAP || nip < 0 || p.row_nnz == nullptr) {
@@ -525,7 +530,7 @@ __global__ __launch_bounds__(THREADS) void k_esc_cta(ProductArgs p) {
     const int tid = threadIdx.x;
     const int row = p.rows[blockIdx.x];
     const int c0 = p.c_rpt[row];
-    const int nip = p.c_rpt[row + 1] - c0;  // the row's NIP-sized slot
+    const int nip = slot_entries(p, row, c0);
     if (nip <= SKIP_LE || (SKIP_GT && nip > NMAX && p.row_nnz != nullptr)) return;
     if (nip > NMAX || p.row_nnz == nullptr) {
         if (tid == 0) report(p.status, kStCapacity, row, nip);
@@ -702,7 +707,7 @@ __global__ __launch_bounds__(THREADS) void k_s2n_cta(ProductArgs p) {
     const int row = p.rows[blockIdx.x];
     const int c0 = p.c_rpt[row];
     // the row's exact nnz, or in one-pass mode its NIP (an upper bound)
-    const int bound = p.c_rpt[row + 1] - c0;
+    const int bound = slot_entries(p, row, c0);
     if (bound > CAP) {
         if (threadIdx.x == 0) report(p.status, kStCapacity, row, bound);
         return;
@@ -806,7 +811,7 @@ __global__ __launch_bounds__(THREADS) void k_s2n_bitmap(ProductArgs p) {
         const int row = p.rows[rid];
         const int c0 = p.c_rpt[row];
         // the row's exact nnz, or in one-pass mode its NIP (an upper bound)
-        const int bound = p.c_rpt[row + 1] - c0;
+        const int bound = slot_entries(p, row, c0);
         if (bound > CAP) {  // uniform over the CTA
             if (tid == 0) report(p.status, kStCapacity, row, bound);
             continue;
@@ -928,7 +933,7 @@ __global__ __launch_bounds__(THREADS) void k_s2n_bitmap_cluster(ProductArgs p) {
         const int row = p.rows[rid];
         const int c0 = p.c_rpt[row];
         // the row's exact nnz, or in one-pass mode its NIP (an upper bound)
-        const int bound = p.c_rpt[row + 1] - c0;
+        const int bound = slot_entries(p, row, c0);
         const int a0 = p.a_rpt[row];
         const int a1 = p.a_rpt[row + 1];
         // 1. bits, each in the CTA that owns its column
@@ -1036,7 +1041,7 @@ __global__ __launch_bounds__(THREADS) void k_s2n_global(ProductArgs p) {
         const int row = p.rows[rid];
         const int c0 = p.c_rpt[row];
         // the row's exact nnz, or in one-pass mode its NIP (an upper bound)
-        const int bound = p.c_rpt[row + 1] - c0;
+        const int bound = slot_entries(p, row, c0);
         const int a0 = p.a_rpt[row];
         const int a1 = p.a_rpt[row + 1];
         const int2 win = cta_col_window<THREADS>(p.a_col, p.b_rpt, p.b_col, a0, a1, p.n_cols, sc);
@@ -1139,13 +1144,9 @@ cudaError_t launch_esc_cta(const ProductArgs& p, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-// The 256-thread ESC bin split by row size: rows of more than kEscCtaSmall
-// products with 256 threads, the others with 128 (half the fixed cost of each
-// radix pass and scan, twice the CTAs per SM).  Both grids cover the whole
-// row list; a CTA whose row belongs to the other kernel returns at once.
-// (1M power-law product: the bin 0.233 -> 0.223 ms serialised.)
-constexpr int kEscCtaSmall = 1024;
-
+// The 256-thread ESC bin's two kernels over one row list: both grids cover the
+// whole list, and a CTA whose row belongs to the other kernel returns at once
+// (so the slot sizes must not be overwritten by the fill: row_slot is null).
 template<typename V>
 cudaError_t launch_esc_cta_split(const ProductArgs& p, cudaStream_t s) {
     k_esc_cta<V, 256, 3072, kEscCtaSmall, false>
@@ -1176,6 +1177,7 @@ constexpr int kSizeBuckets = 2048;
 __global__ __launch_bounds__(kSortThreads) void k_rows_largest_first(int32_t* __restrict__ rows,
                                                                      int32_t n,
                                                                      const int32_t* __restrict__ c_rpt,
+                                                                     const int32_t* __restrict__ row_slot,
                                                                      int32_t* __restrict__ work) {
     constexpr int PER = kSizeBuckets / kSortThreads;
     __shared__ int32_t s_count[kSizeBuckets];  // per bucket: count, then first slot
@@ -1187,7 +1189,7 @@ __global__ __launch_bounds__(kSortThreads) void k_rows_largest_first(int32_t* __
     __syncthreads();
     // descending: bucket 0 holds the largest rows
     auto bucket = [&](int r) {
-        const int size = c_rpt[r + 1] - c_rpt[r];
+        const int size = row_slot != nullptr ? row_slot[r] : c_rpt[r + 1] - c_rpt[r];
         return kSizeBuckets - 1 - min(size >> 5, kSizeBuckets - 1);
     };
     for (int i = tid; i < n; i += kSortThreads) atomicAdd(&s_count[bucket(rows[i])], 1);
@@ -1226,7 +1228,7 @@ cudaError_t launch_bitmap(const ProductArgs& p, cudaStream_t s) {
         // the sort kernel also zeroes the row counter
         if (p.nrows > grid && p.nrows <= kSortRowsMax) {
             k_rows_largest_first<<<1, kSortThreads, 0, s>>>(const_cast<int32_t*>(p.rows),
-                                                            p.nrows, p.c_rpt, p.work);
+                                                            p.nrows, p.c_rpt, p.row_slot, p.work);
             if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
         } else if (cudaError_t e = cudaMemsetAsync(p.work, 0, sizeof(int32_t), s);
                    e != cudaSuccess) {
@@ -1384,6 +1386,18 @@ const BinLauncher EscSplitBin<V>::entry = {BinKind::Team, kEscSplit, 8, 256,
                                            "esc_team32_n512", launch_esc<V, 32, 256, kEscSplit>};
 
 template<typename V>
+struct EscCtaBins {
+    static const BinLauncher entries[2];
+};
+template<typename V>
+const BinLauncher EscCtaBins<V>::entries[2] = {
+    {BinKind::Cta, kEscCtaSmall, 1, 128, EscCtaLayout<V, 128, kEscCtaSmall>::bytes,
+     "esc_cta128_n1024", launch_esc_cta<V, 128, kEscCtaSmall>},
+    {BinKind::Cta, 3072, 1, 256, EscCtaLayout<V, 256, 3072>::bytes, "esc_cta256_n3072",
+     launch_esc_cta<V, 256, 3072>},
+};
+
+template<typename V>
 cudaError_t prepare_one() {
     cudaError_t e = cudaSuccess;
 #define B200_SMEM(kern, bytes)                                                            \
@@ -1402,6 +1416,7 @@ cudaError_t prepare_one() {
     B200_SMEM((k_esc_team<V, 32, 256, 768>), (EscLayout<V, 32, 256, 768>::bytes));
     B200_SMEM((k_esc_team<V, 32, 256, kEscSplit>), (EscLayout<V, 32, 256, kEscSplit>::bytes));
     B200_SMEM((k_esc_cta<V, 256, 3072>), (EscCtaLayout<V, 256, 3072>::bytes));
+    B200_SMEM((k_esc_cta<V, 128, kEscCtaSmall>), (EscCtaLayout<V, 128, kEscCtaSmall>::bytes));
     B200_SMEM((k_esc_cta<V, 256, 3072, kEscCtaSmall, false>), (EscCtaLayout<V, 256, 3072>::bytes));
     B200_SMEM((k_esc_cta<V, 128, kEscCtaSmall, 0, true>), (EscCtaLayout<V, 128, kEscCtaSmall>::bytes));
 #undef B200_SMEM
@@ -1442,6 +1457,8 @@ int s2n_esc_ladder_f32(const BinLauncher** out) {
 
 const BinLauncher* s2n_esc_split_bin_f64() { return &EscSplitBin<double>::entry; }
 const BinLauncher* s2n_esc_split_bin_f32() { return &EscSplitBin<float>::entry; }
+const BinLauncher* s2n_esc_cta_f64(int which) { return &EscCtaBins<double>::entries[which]; }
+const BinLauncher* s2n_esc_cta_f32(int which) { return &EscCtaBins<float>::entries[which]; }
 
 cudaError_t launch_esc_sample(const ProductArgs& p, int32_t m, int32_t samples,
                               const EscLimits& lim, EscSample* out, cudaStream_t s) {

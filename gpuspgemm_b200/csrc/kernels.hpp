@@ -62,6 +62,10 @@ struct ProductArgs {
     // bound); the kernel writes the row's exact nnz here (nullptr: c_rpt is
     // C's exact row pointer)
     int32_t* row_nnz;
+    // one-pass fill: the entries of each row's slot, where the slots are not
+    // in row order (nullptr: c_rpt[row + 1] - c_rpt[row]).  It may be row_nnz
+    // itself: a row is read and then written by the one kernel that fills it.
+    const int32_t* row_slot;
     // SMs of the device (persistent kernels size their grid by it; 0: 148)
     int32_t sm_count;
     // persistent bins: a device counter the CTAs take their next row from
@@ -108,6 +112,13 @@ int s2n_esc_ladder_f32(const BinLauncher** out);
 // (rows of at most kEscSplit products: a smaller kernel, more CTAs per SM).
 const BinLauncher* s2n_esc_split_bin_f64();
 const BinLauncher* s2n_esc_split_bin_f32();
+// The 256-thread bin's two kernels where its rows come in two lists: rows of
+// at most kEscCtaSmall products on 128 threads (which = 0), the others on 256
+// (half the fixed cost of each radix pass and scan, twice the CTAs per SM:
+// 1M power-law product, the bin 0.233 -> 0.223 ms serialised).
+constexpr int kEscCtaSmall = 1024;
+const BinLauncher* s2n_esc_cta_f64(int which);
+const BinLauncher* s2n_esc_cta_f32(int which);
 
 // Sampled compression of the first kEscBins fill bins of a one-pass product:
 // the NIP and exact nnz of up to `samples` rows spread evenly over A, summed
@@ -179,12 +190,28 @@ cudaError_t launch_nip_hist(const int32_t* a_rpt, const int32_t* a_col, const in
 // limits include every limit of the final ladder (dlad when given, else lad):
 // the outputs of launch_bin_offsets for the final ladder, all bins at once,
 // except that hist (another array) receives offsets within each bin: the
-// scatter that reads them is launched with bin_relative.  It also zeroes
-// zero[0..nzero), words a later kernel needs cleared.
+// scatter that reads them is launched with bin_relative.
 cudaError_t launch_bin_offsets_map(const int32_t* src_hist, int32_t* hist, int32_t nctas,
                                    const Ladder& src, int64_t* cta_sum, Plan* plan,
-                                   const Ladder& lad, const Ladder* dlad, cudaStream_t s,
-                                   unsigned long long* zero = nullptr, int32_t nzero = 0);
+                                   const Ladder& lad, const Ladder* dlad, cudaStream_t s);
+// Append binning, one launch a pass (rows into per-bin lists: bin b's rows at
+// lists[b * stride ...], stride >= m, their number in plan->bin_size[b]; the
+// plan zeroed by the caller receives the keys' total and max).  Used up to
+// kAppendMaxRows rows: the lists take kListBins words a row.
+constexpr int32_t kAppendMaxRows = int32_t(1) << 22;
+constexpr int kListBins = 11;
+// key = NIP, written to c_rpt; off (or nullptr) receives each row's slot start
+cudaError_t launch_nip_append(const int32_t* a_rpt, const int32_t* a_col, const int32_t* b_rpt,
+                              int32_t m, int32_t* c_rpt, int32_t* off, int32_t* lists,
+                              int64_t stride, Plan* plan, DevStatus* st, const Ladder& lad,
+                              cudaStream_t s);
+// keys in memory
+cudaError_t launch_key_append(const int32_t* keys, int32_t m, int32_t* off, int32_t* lists,
+                              int64_t stride, Plan* plan, const Ladder& lad, cudaStream_t s);
+// launch_rpt_scan1 (below) that also appends the rows, keyed by their counts
+cudaError_t launch_rpt_scan_append(int32_t* cnt, int32_t m, unsigned long long* state, Plan* plan,
+                                   DevStatus* st, int32_t* lists, int64_t stride,
+                                   const Ladder& lad, cudaStream_t s);
 // Pass 1' (key = nnz already in c_rpt): per-CTA sums and bin histograms.
 // dlad: limits chosen on the device (same bin count as lad), or nullptr.
 cudaError_t launch_nnz_hist(const int32_t* c_rpt, int32_t m, int32_t* hist, int64_t* cta_sum,
@@ -208,7 +235,9 @@ cudaError_t launch_bin_scatter(int32_t* c_rpt, int32_t m, const int32_t* hist_of
 // too long reports kStWait in st.  Used for rpt_scan_tiles(m) <=
 // kScanMaxTiles (the size of the state in the scratch).
 constexpr int kScanTile = 4096;
-constexpr int kScanMaxTiles = 2048;
+constexpr int kScanAppendTile = 1024;  // of the scan that also appends
+constexpr int kScanMaxTiles = 4096;
+static_assert(kAppendMaxRows <= int64_t(kScanAppendTile) * kScanMaxTiles, "scan state");
 inline int rpt_scan_tiles(int32_t m) { return (m + kScanTile - 1) / kScanTile; }
 cudaError_t launch_rpt_scan1(int32_t* cnt, int32_t m, unsigned long long* state, Plan* plan,
                              DevStatus* st, cudaStream_t s);

@@ -57,8 +57,8 @@ constexpr int64_t kBitmapBudget = int64_t(1) << 30;
 struct Scratch {
     DevStatus* status;
     Plan* plan1;
-    // the one-pass row pointer's look-back: a ticket counter and one state per
-    // tile (behind the mirrored front)
+    // the row pointer's look-back: a ticket counter and one state per tile
+    // (behind the mirrored front, zeroed with it)
     unsigned long long* scan_state;
     Plan* plan2;
     int32_t* hist1;
@@ -196,15 +196,18 @@ spgemm_status ensure_scratch(spgemm_handle_s* h, int32_t m, Scratch* s, cudaStre
     const size_t o_fail_count = take(sizeof(int32_t));
     const size_t o_sample = take(sizeof(EscSample));
     const size_t o_dladder = take(sizeof(Ladder));
+    const size_t o_scan = take(sizeof(unsigned long long) * (1 + kScanMaxTiles));
     const size_t o_hist1 = take(sizeof(int32_t) * kMaxBins * nctas);
     const size_t o_hist2 = take(sizeof(int32_t) * kMaxBins * nctas);
     const size_t o_hist3 = take(sizeof(int32_t) * kMaxBins * nctas);
     const size_t o_sum = take(sizeof(int64_t) * nctas);
-    const size_t o_bins1 = take(sizeof(int32_t) * mm);
-    const size_t o_bins2 = take(sizeof(int32_t) * mm);
+    // append binning: one region of per-bin lists serves the passes in turn
+    // (each pass's lists are read before the next pass starts)
+    const bool append = m <= kAppendMaxRows;
+    const size_t o_bins1 = take(sizeof(int32_t) * mm * (append ? kListBins : 1));
+    const size_t o_bins2 = append ? o_bins1 : take(sizeof(int32_t) * mm);
     const size_t o_fail = take(sizeof(int32_t) * mm);
     const size_t o_work = take(sizeof(int32_t) * kMaxBins);
-    const size_t o_scan = take(sizeof(unsigned long long) * (1 + kScanMaxTiles));
     if (spgemm_status st = regrow(h, &h->scratch, &h->scratch_bytes, off + off / 4, stream);
         st != SPGEMM_OK)
         return st;
@@ -261,14 +264,15 @@ Ladder make_ladder(const BinLauncher* bins, int nb, int min_bin) {
     return l;
 }
 
-spgemm_status fork_streams(spgemm_handle_s* h, cudaStream_t main) {
+// The first n side streams wait for main, and main for them.
+spgemm_status fork_streams(spgemm_handle_s* h, cudaStream_t main, int n) {
     B200_TRY(cudaEventRecord(h->ev_fork, main));
-    for (int i = 0; i < h->nside; i++) B200_TRY(cudaStreamWaitEvent(h->side[i], h->ev_fork, 0));
+    for (int i = 0; i < n; i++) B200_TRY(cudaStreamWaitEvent(h->side[i], h->ev_fork, 0));
     return SPGEMM_OK;
 }
 
-spgemm_status join_streams(spgemm_handle_s* h, cudaStream_t main) {
-    for (int i = 0; i < h->nside; i++) {
+spgemm_status join_streams(spgemm_handle_s* h, cudaStream_t main, int n) {
+    for (int i = 0; i < n; i++) {
         B200_TRY(cudaEventRecord(h->ev_join[i], h->side[i]));
         B200_TRY(cudaStreamWaitEvent(main, h->ev_join[i], 0));
     }
@@ -320,7 +324,7 @@ spgemm_status status_to_error(const DevStatus& st) {
 // the front.
 spgemm_status mirror_start(spgemm_handle_s* h, cudaStream_t stream, const Scratch& s) {
     const char* dev0 = static_cast<const char*>(h->scratch);
-    const size_t front = static_cast<size_t>(reinterpret_cast<const char*>(s.hist1) - dev0);
+    const size_t front = static_cast<size_t>(reinterpret_cast<const char*>(s.scan_state) - dev0);
     if (front > kFrontBytes) return fail(SPGEMM_ERR_INTERNAL, "scratch front exceeds its mirror");
     cudaStream_t copy = h->side[kMaxSide - 1];
     B200_TRY(cudaEventRecord(h->ev_front, stream));
@@ -350,7 +354,7 @@ spgemm_status sync_mirror(spgemm_handle_s* h, cudaStream_t stream, const Plan* p
                           const Scratch& s, bool with_sample = false,
                           const Plan* plan_b = nullptr) {
     const char* dev0 = static_cast<const char*>(h->scratch);
-    const size_t front = static_cast<size_t>(reinterpret_cast<const char*>(s.hist1) - dev0);
+    const size_t front = static_cast<size_t>(reinterpret_cast<const char*>(s.scan_state) - dev0);
     if (front > kFrontBytes) return fail(SPGEMM_ERR_INTERNAL, "scratch front exceeds its mirror");
     B200_TRY(cudaMemcpyAsync(h->front_host, h->scratch, front, cudaMemcpyDeviceToHost, stream));
     B200_TRY(cudaStreamSynchronize(stream));
@@ -421,11 +425,18 @@ void resolve_profile(spgemm_handle_s* h) {
 }
 
 // One kernel per non-empty bin, heavy bins first, round-robin over the side
-// streams (forked from and joined back into `main`).
+// streams (forked from and joined back into `main`).  ids: the bins' numbers
+// in the profile (nullptr: their indices).
 spgemm_status launch_bins(spgemm_handle_s* h, const BinLauncher* bins, int nb, int phase,
                           const Plan& plan, const int32_t* row_lists, const ProductArgs& base,
-                          cudaStream_t main) {
-    if (spgemm_status st = fork_streams(h, main); st != SPGEMM_OK) return st;
+                          cudaStream_t main, const int* ids = nullptr) {
+    int filled = 0;
+    for (int b = 0; b < nb; b++) filled += plan.bin_size[b] > 0;
+    // one bin needs no side stream, and n bins no more than n of them: each
+    // costs three calls (~2 us) that a small product waits for
+    const int nside = filled <= 1 ? 0 : std::min(h->nside, filled);
+    if (nside > 0)
+        if (spgemm_status st = fork_streams(h, main, nside); st != SPGEMM_OK) return st;
     // the heaviest non-empty bin (the first launched) has side stream 0 --
     // the high-priority one -- to itself: it is the phase's longest kernel,
     // and nothing queues behind it; the others share the remaining streams
@@ -437,15 +448,16 @@ spgemm_status launch_bins(spgemm_handle_s* h, const BinLauncher* bins, int nb, i
         a.rows = row_lists + plan.bin_off[b];
         a.nrows = rows;
         a.work = base.work != nullptr ? base.work + b : nullptr;
-        cudaStream_t s = h->side[next == 0 || h->nside == 1 ? 0 : 1 + (next - 1) % (h->nside - 1)];
+        cudaStream_t s = nside == 0 ? main
+                                    : h->side[next == 0 || nside == 1 ? 0 : 1 + (next - 1) % (nside - 1)];
         next++;
         const BinLauncher& L = bins[b];
-        if (spgemm_status st = timed(h, L.name, phase, b, rows, s,
+        if (spgemm_status st = timed(h, L.name, phase, ids != nullptr ? ids[b] : b, rows, s,
                                      [&](cudaStream_t ss) { return L.launch(a, ss); });
             st != SPGEMM_OK)
             return st;
     }
-    return join_streams(h, main);
+    return join_streams(h, main, nside);
 }
 
 // Plan capture request for product(): the team fill bins' routing limits are
@@ -461,6 +473,46 @@ struct CaptureReq {
     bool launch_now = true;
     cudaGraph_t graph = nullptr;
 };
+
+// Append binning's row lists: bin b's at b * m (the device only counts rows).
+void list_offsets(Plan* plan, int nb, int32_t m) {
+    for (int b = 0; b < nb; b++) plan->bin_off[b] = b * m;
+}
+
+// The limits append binning counts one-pass rows by: the fill ladder's, and,
+// where the fill may expand, sort and compress, kEscSplit and kEscCtaSmall
+// too.  Which kernel takes which list is decided when the sample is known:
+// src[e] is the fill bin limit e comes from (kFromSplit, kFromSmall: inserted).
+constexpr int kFromSplit = -1;
+constexpr int kFromSmall = -2;
+struct ListLadder {
+    Ladder lad;
+    int src[kMaxBins];
+    // the fill bin that list e belongs to
+    int fill_bin(int e, bool split) const {
+        if (src[e] == kFromSplit) return kEscBins - 1;
+        if (src[e] == kFromSmall) return kEscBins;
+        return split && src[e] == kEscBins - 1 ? kEscBins : src[e];
+    }
+};
+
+ListLadder list_ladder(const Ladder& fill, bool esc) {
+    ListLadder l = {};
+    int nb = 0;
+    for (int b = 0; b < fill.nb; b++) {
+        auto put = [&](int32_t limit, int from) {
+            l.lad.limit[nb] = limit;
+            l.src[nb++] = from;
+        };
+        if (esc && b == kEscBins - 1) put(kEscSplit, kFromSplit);
+        if (esc && b == kEscBins) put(kEscCtaSmall, kFromSmall);
+        put(fill.limit[b], b);
+        // rows forced to bin min_bin or above: to the lists past the bin below
+        if (b == fill.min_bin - 1) l.lad.min_bin = nb;
+    }
+    l.lad.nb = nb;
+    return l;
+}
 
 Ladder scaled_ladder(const BinLauncher* bins, int nb, int min_bin, double team_scale,
                      double cta_scale = 1.0) {
@@ -581,6 +633,8 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
 
     // ---- count pass: NIP per row and bins ---------------------------------
     const int nctas = bin_ctas(m);
+    // one launch per binning pass, a row list per bin (k_bin.cu)
+    const bool append = m <= kAppendMaxRows;
     const Ladder lad1 = make_ladder(sym, nsym, h->min_sym_bin);
     // Compression sample (products that may run one pass): it reads A and B
     // only, so it runs on a side stream beside the NIP pass (forked before
@@ -610,9 +664,10 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
         B200_STEP(timed(h, "esc_sample", 0, -1, samples, side, [&](cudaStream_t ss) {
             return launch_esc_sample(ps, m, samples, el, s.sample, ss);
         }));
-        B200_STEP(timed(h, "esc_decide", 0, -1, 1, side, [&](cudaStream_t ss) {
-            return launch_esc_decide(s.sample, ladf, esc_mode, s.dladder, ss);
-        }));
+        if (!append)  // (append binning needs no decision on the device)
+            B200_STEP(timed(h, "esc_decide", 0, -1, 1, side, [&](cudaStream_t ss) {
+                return launch_esc_decide(s.sample, ladf, esc_mode, s.dladder, ss);
+            }));
         if (cudaError_t e = cudaEventRecord(h->ev_sample, side); e != cudaSuccess)
             return bail(cuda_fail(e, "join the sample stream"));
     }
@@ -654,28 +709,41 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
             }
         }
     }
-    const bool nip_counts_fill = early && ladx_ok;
+    const ListLadder lists = list_ladder(ladf, esc_mode != 2);
+    const bool nip_counts_fill = !append && early && ladx_ok;
     bool mirror_pending = false;  // mirror_start ran: the first wait is on its event
-    // the row pointer's look-back scan needs its ticket and tile states zeroed
+    // (the row pointer's look-back scan runs once per product: its state was
+    // zeroed with the scratch front)
     const bool scan1 = rpt_scan_tiles(m) <= kScanMaxTiles;
-    const size_t scan_bytes = sizeof(unsigned long long) * (1 + size_t(rpt_scan_tiles(m)));
-    bool scan_zeroed = false;
+    // the plan that receives the fill bins of a one-pass product
+    Plan* const fill_plan = append && early ? s.plan1 : s.plan2;
     B200_STEP(timed(h, "nip_hist", 0, -1, m, stream, [&](cudaStream_t ss) {
+        if (append)
+            return launch_nip_append(A->rpt, A->col, B->rpt, m, c_rpt, off, s.bins1, m, s.plan1,
+                                     s.status, early ? lists.lad : lad1, ss);
         return launch_nip_hist(A->rpt, A->col, B->rpt, m, c_rpt, off, s.hist1, s.plan1, s.status,
                                lad1, ss, s.hist3, s.cta_sum, nip_counts_fill ? &ladx : nullptr);
     }));
     auto fill_binning = [&]() -> spgemm_status {
+        if (append) {
+            if (sampled) B200_TRY(cudaStreamWaitEvent(stream, h->ev_sample, 0));
+            if (early) return SPGEMM_OK;  // the NIP pass binned the rows
+            B200_STEP_R(regrow(h, &h->slots, &h->slots_bytes, sizeof(int32_t) * (size_t(m) + 1),
+                               stream));
+            off = static_cast<int32_t*>(h->slots);
+            B200_STEP_R(timed(h, "nip_fill_bins", 2, -1, m, stream, [&](cudaStream_t ss) {
+                return launch_key_append(c_rpt, m, off, s.bins2, m, s.plan2, lists.lad, ss);
+            }));
+            return SPGEMM_OK;
+        }
         if (nip_counts_fill) {
             // the NIP pass counted the rows by ladx: offsets for the chosen
             // ladder, then the scatter
             if (sampled) B200_TRY(cudaStreamWaitEvent(stream, h->ev_sample, 0));
-            // (the row pointer's look-back state is zeroed by the same launch)
             B200_STEP_R(timed(h, "nip_fill_offsets", 2, -1, m, stream, [&](cudaStream_t ss) {
                 return launch_bin_offsets_map(s.hist3, s.hist2, nctas, ladx, s.cta_sum, s.plan2,
-                                              ladh, dlad, ss, scan1 ? s.scan_state : nullptr,
-                                              scan1 ? static_cast<int32_t>(scan_bytes / 8) : 0);
+                                              ladh, dlad, ss);
             }));
-            scan_zeroed = scan1;
             // everything the host decides on is final here (the NIP pass's
             // plan, the fill plan, the sample, the status): its copy goes
             // ahead of the scatter, which then overlaps the host's wait
@@ -710,6 +778,13 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     };
     // The count binning by NIP (the two-pass path's).
     auto count_binning = [&]() -> spgemm_status {
+        if (append) {
+            if (early)  // the NIP pass binned for the fill (plan1); plan2 is still clear
+                B200_STEP_R(timed(h, "nip_count_bins", 0, -1, m, stream, [&](cudaStream_t ss) {
+                    return launch_key_append(c_rpt, m, nullptr, s.bins1, m, s.plan2, lad1, ss);
+                }));
+            return SPGEMM_OK;
+        }
         B200_STEP_R(timed(h, "bin_offsets", 0, -1, m, stream, [&](cudaStream_t ss) {
             return launch_bin_offsets(s.hist1, nctas, nullptr, s.plan1, lad1, ss);
         }));
@@ -726,15 +801,16 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     }
     mark(0);
     if (mirror_pending) {
-        B200_STEP(mirror_finish(h, s.plan1, s, early && sampled, early ? s.plan2 : nullptr));
+        B200_STEP(mirror_finish(h, s.plan1, s, early && sampled, early ? fill_plan : nullptr));
     } else {
-        B200_STEP(sync_mirror(h, stream, s.plan1, s, early && sampled, early ? s.plan2 : nullptr));
+        B200_STEP(sync_mirror(h, stream, s.plan1, s, early && sampled, early ? fill_plan : nullptr));
     }
     mark(1);
     B200_STEP(status_to_error(h->mirror->status));
     Plan p1 = h->mirror->plan;  // bin sizes valid once the count binning ran
     h->info.nip = p1.total_key;
     h->info.max_row_nip = p1.max_key;
+    if (append) list_offsets(&p1, nsym, m);
     bool counted = !early;
     if (counted)
         for (int b = 0; b < nsym && b < 16; b++) h->info.sym_bin_rows[b] = p1.bin_size[b];
@@ -808,8 +884,9 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
         }
         mark(3);
         B200_ONE(status_to_error(h->mirror->status));
-        const Plan pf = h->mirror->plan_b;
+        Plan pf = h->mirror->plan_b;
         const EscSample es = h->mirror->sample;
+        if (append) list_offsets(&pf, lists.lad.nb, m);
         // sampled: the NIP of rows above the team bins, the team bins' NIP/nnz
         int64_t team_nip = 0;
         int64_t team_nnz = 0;
@@ -839,12 +916,19 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
         // C.rpt receives each row's exact nnz from the fill kernel of its bin;
         // a row without products keeps the NIP of 0 the NIP pass wrote there
         // (and the scan writes C.rpt[m])
+        // the largest team bin and the 256-thread bin follow one decision,
+        // which also moves the split of their limits (append binning has
+        // counted by both splits; else the device decided before it binned)
+        const bool split =
+            esc_ok && (esc_mode == 1 ||
+                       (sampled && (append ? es.nnz[kEscBins - 1] > 0 &&
+                                                 static_cast<double>(es.nip[kEscBins - 1]) <=
+                                                     kEscMaxRatio[kEscBins - 1] *
+                                                         static_cast<double>(es.nnz[kEscBins - 1])
+                                           : es.split != 0)));
         if (esc_ok) {
             const BinLauncher* esc = nullptr;
             const int nesc = sizeof(V) == 8 ? s2n_esc_ladder_f64(&esc) : s2n_esc_ladder_f32(&esc);
-            // the largest team bin and the 256-thread bin follow the device's
-            // decision (which also moved the split of their limits)
-            const bool split = esc_mode == 1 || (sampled && es.split != 0);
             for (int b = 0; b < kEscLadderBins && b < nesc && b < nfil; b++) {
                 const bool use =
                     b >= kEscBins - 1
@@ -862,28 +946,51 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
                 }
             }
         }
-        for (int b = 0; b < nfil && b < 16; b++) h->info.num_bin_rows[b] = pf.bin_size[b];
+        // append binning: the kernel of each list
+        BinLauncher list_fil[kMaxBins];
+        int list_ids[kMaxBins];
+        if (append) {
+            for (int e = 0; e < lists.lad.nb; e++) {
+                const int b = lists.fill_bin(e, split);
+                list_ids[e] = b;
+                list_fil[e] = one_fil[b];
+                if (b == kEscBins && split) {
+                    const int which = lists.lad.limit[e] <= kEscCtaSmall ? 0 : 1;
+                    list_fil[e] = sizeof(V) == 8 ? *s2n_esc_cta_f64(which) : *s2n_esc_cta_f32(which);
+                }
+                h->info.num_bin_rows[b] += pf.bin_size[e];
+            }
+        } else {
+            for (int b = 0; b < nfil && b < 16; b++) h->info.num_bin_rows[b] = pf.bin_size[b];
+        }
+        const BinLauncher* fill_bins = append ? list_fil : one_fil;
+        const int nfill = append ? lists.lad.nb : nfil;
         pa.c_rpt = off;
         pa.c_col = tmp_col;
         pa.c_val = tmp_val;
         pa.row_nnz = c_rpt;
-        if (const int32_t gr = global_bitmap_rows(fil, nfil, pf, n); gr > 0) {
+        // append binning's slots are not in row order: a row's slot size is the
+        // NIP that C.rpt holds until the row's fill kernel writes its nnz there
+        pa.row_slot = append ? c_rpt : nullptr;
+        if (const int32_t gr = global_bitmap_rows(fill_bins, nfill, pf, n); gr > 0) {
             int32_t nmaps = 0;
             B200_ONE(ensure_bitmaps(h, pa.words, gr, &nmaps, stream));
             pa.bitmaps = h->bitmaps;
             pa.nmaps = nmaps;
         }
         mark(4);
-        B200_ONE(launch_bins(h, one_fil, nfil, 3, pf, s.bins2, pa, stream));
-        // row pointer from the counts, into the count binning's plan (reset:
-        // its max and overflow only ever grow): one look-back scan -- or, past
-        // its tile limit, a one-bin pass of the binning kernels
-        B200_ONE_CUDA(cudaMemsetAsync(s.plan1, 0, sizeof(Plan), stream), "reset a plan");
-        if (scan1 && !scan_zeroed)
-            B200_ONE_CUDA(cudaMemsetAsync(s.scan_state, 0, scan_bytes, stream), "reset the scan");
+        B200_ONE(launch_bins(h, fill_bins, nfill, 3, pf, s.bins2, pa, stream,
+                             append ? list_ids : nullptr));
+        // row pointer from the counts, into the plan the fill bins do not use
+        // (reset if a pass has written it: its max and overflow only ever
+        // grow): one look-back scan -- or, past its tile limit, a one-bin pass
+        // of the binning kernels
+        Plan* const rpt_plan = fill_plan == s.plan1 ? s.plan2 : s.plan1;
+        if (rpt_plan == s.plan1)
+            B200_ONE_CUDA(cudaMemsetAsync(s.plan1, 0, sizeof(Plan), stream), "reset a plan");
         if (scan1) {
             B200_ONE(timed(h, "count_scan_rows", 2, -1, m, stream, [&](cudaStream_t ss) {
-                return launch_rpt_scan1(c_rpt, m, s.scan_state, s.plan1, s.status, ss);
+                return launch_rpt_scan1(c_rpt, m, s.scan_state, rpt_plan, s.status, ss);
             }));
         } else {
             Ladder one = {};
@@ -929,7 +1036,7 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
                 C->col = nullptr;
                 C->val = nullptr;
             };
-            if (spgemm_status st = sync_mirror(h, stream, s.plan1, s); st != SPGEMM_OK)
+            if (spgemm_status st = sync_mirror(h, stream, rpt_plan, s); st != SPGEMM_OK)
                 return drop_c(), bail(st);
             if (spgemm_status st = status_to_error(h->mirror->status); st != SPGEMM_OK)
                 return drop_c(), bail(st);
@@ -977,7 +1084,7 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
             resolve_profile(h);
             return SPGEMM_OK;
         }
-        B200_ONE(sync_mirror(h, stream, s.plan1, s));
+        B200_ONE(sync_mirror(h, stream, rpt_plan, s));
         B200_ONE(status_to_error(h->mirror->status));
         const Plan pc = h->mirror->plan;
         if (pc.overflow || pc.total_key > nip_total)
@@ -1016,17 +1123,29 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
         if (cudaError_t e = cudaStreamWaitEvent(stream, h->ev_sample, 0); e != cudaSuccess)
             return bail(cuda_fail(e, "join the sample stream"));
     }
+    // the scan pass's plan: the one the fill binning by NIP used, if it ran
+    Plan* const scan_plan = fill_plan;
     if (early || one_pass) {
-        // the fill binning by NIP ran: its plan is reused by the scan pass
-        if (cudaError_t e = cudaMemsetAsync(s.plan2, 0, sizeof(Plan), stream); e != cudaSuccess)
+        if (cudaError_t e = cudaMemsetAsync(scan_plan, 0, sizeof(Plan), stream); e != cudaSuccess)
             return bail(cuda_fail(e, "reset a plan"));
     }
-    if (!counted) {
-        // a product binned early for one pass runs two: its count binning now
-        B200_STEP(count_binning());
-        B200_STEP(sync_mirror(h, stream, s.plan1, s));
+    if (!counted || (append && one_pass)) {
+        // a product binned for a one-pass fill runs two passes: its count
+        // binning now (again, where the lists of the fill bins overwrote it)
+        Plan* const count_plan = append && early ? s.plan2 : s.plan1;
+        if (append && !early) {
+            if (cudaError_t e = cudaMemsetAsync(s.plan1, 0, sizeof(Plan), stream); e != cudaSuccess)
+                return bail(cuda_fail(e, "reset a plan"));
+            B200_STEP(timed(h, "nip_count_bins", 0, -1, m, stream, [&](cudaStream_t ss) {
+                return launch_key_append(c_rpt, m, nullptr, s.bins1, m, s.plan1, lad1, ss);
+            }));
+        } else {
+            B200_STEP(count_binning());
+        }
+        B200_STEP(sync_mirror(h, stream, count_plan, s));
         B200_STEP(status_to_error(h->mirror->status));
         p1 = h->mirror->plan;
+        if (append) list_offsets(&p1, nsym, m);
         for (int b = 0; b < nsym && b < 16; b++) h->info.sym_bin_rows[b] = p1.bin_size[b];
     }
 
@@ -1043,9 +1162,14 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     }
     // cluster bin, then its spills, then knob-forced global rows: one chain on
     // the first side stream; the other bins round-robin on the rest
-    B200_STEP(fork_streams(h, stream));
+    int sym_filled = 0;
+    for (int b = 0; b < clus1; b++) sym_filled += p1.bin_size[b] > 0;
+    const bool chain_used = cluster_rows > 0 || global_rows > 0;
+    const int sym_side =
+        sym_filled + (chain_used ? 1 : 0) <= 1 ? 0 : std::min(h->nside, sym_filled + (chain_used ? 1 : 0));
+    if (sym_side > 0) B200_STEP(fork_streams(h, stream, sym_side));
     {
-        cudaStream_t chain = h->side[0];
+        cudaStream_t chain = sym_side > 0 ? h->side[0] : stream;
         if (cluster_rows > 0) {
             ProductArgs a = pa;
             a.rows = s.bins1 + p1.bin_off[clus1];
@@ -1068,8 +1192,7 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
             B200_STEP(timed(h, sym[glob1].name, 1, glob1, global_rows, chain,
                             [&](cudaStream_t ss) { return sym[glob1].launch(a, ss); }));
         }
-        const bool chain_used = cluster_rows > 0 || global_rows > 0;
-        const int first = chain_used && h->nside > 1 ? 1 : 0;
+        const int first = chain_used && sym_side > 1 ? 1 : 0;
         int next = first;
         for (int b = clus1 - 1; b >= 0; b--) {
             const int rows = p1.bin_size[b];
@@ -1077,31 +1200,39 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
             ProductArgs a = pa;
             a.rows = s.bins1 + p1.bin_off[b];
             a.nrows = rows;
-            B200_STEP(timed(h, sym[b].name, 1, b, rows, h->side[next],
+            B200_STEP(timed(h, sym[b].name, 1, b, rows, sym_side > 0 ? h->side[next] : stream,
                             [&](cudaStream_t ss) { return sym[b].launch(a, ss); }));
-            next = next + 1 < h->nside ? next + 1 : first;
+            next = next + 1 < sym_side ? next + 1 : first;
         }
     }
-    B200_STEP(join_streams(h, stream));
+    B200_STEP(join_streams(h, stream, sym_side));
 
     // ---- scan pass: row pointer and fill bins -------------------------------
     const Ladder lad2 = scaled_ladder(fil, nfil, h->min_num_bin, cr ? cr->team_scale : 1.0,
                                       cr ? cr->cta_scale : 1.0);
-    B200_STEP(timed(h, "nnz_hist", 2, -1, m, stream, [&](cudaStream_t ss) {
-        return launch_nnz_hist(c_rpt, m, s.hist2, s.cta_sum, s.plan2, lad2, ss);
-    }));
-    B200_STEP(timed(h, "scan_offsets", 2, -1, m, stream, [&](cudaStream_t ss) {
-        return launch_bin_offsets(s.hist2, nctas, s.cta_sum, s.plan2, lad2, ss);
-    }));
-    B200_STEP(timed(h, "scan_scatter", 2, -1, m, stream, [&](cudaStream_t ss) {
-        return launch_bin_scatter(c_rpt, m, s.hist2, s.cta_sum, s.bins2, s.plan2, lad2, true,
-                                  ss);
-    }));
+    if (append) {
+        B200_STEP(timed(h, "scan_bins", 2, -1, m, stream, [&](cudaStream_t ss) {
+            return launch_rpt_scan_append(c_rpt, m, s.scan_state, scan_plan, s.status, s.bins2, m,
+                                          lad2, ss);
+        }));
+    } else {
+        B200_STEP(timed(h, "nnz_hist", 2, -1, m, stream, [&](cudaStream_t ss) {
+            return launch_nnz_hist(c_rpt, m, s.hist2, s.cta_sum, s.plan2, lad2, ss);
+        }));
+        B200_STEP(timed(h, "scan_offsets", 2, -1, m, stream, [&](cudaStream_t ss) {
+            return launch_bin_offsets(s.hist2, nctas, s.cta_sum, s.plan2, lad2, ss);
+        }));
+        B200_STEP(timed(h, "scan_scatter", 2, -1, m, stream, [&](cudaStream_t ss) {
+            return launch_bin_scatter(c_rpt, m, s.hist2, s.cta_sum, s.bins2, s.plan2, lad2, true,
+                                      ss);
+        }));
+    }
     mark(2);
-    B200_STEP(sync_mirror(h, stream, s.plan2, s));
+    B200_STEP(sync_mirror(h, stream, scan_plan, s));
     mark(3);
     B200_STEP(status_to_error(h->mirror->status));
-    const Plan p2 = h->mirror->plan;
+    Plan p2 = h->mirror->plan;
+    if (append) list_offsets(&p2, nfil, m);
     h->info.sym_fail_rows = h->mirror->fail_count;
     if (p2.overflow)
         return bail(fail(SPGEMM_ERR_OVERFLOW,
@@ -1144,10 +1275,18 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
         int32_t* bins = nullptr;
         B200_STEP(plan_alloc(plan, reinterpret_cast<void**>(&bins), sizeof(int32_t) * size_t(m),
                              stream));
-        if (cudaError_t e = cudaMemcpyAsync(bins, s.bins2, sizeof(int32_t) * size_t(m),
-                                            cudaMemcpyDeviceToDevice, stream);
-            e != cudaSuccess)
-            return bail(cuda_fail(e, "copy fill bins"));
+        int32_t at = 0;  // the lists one after another
+        for (int b = 0; b < nfil; b++) {
+            const int32_t rows = p2.bin_size[b];
+            if (rows > 0)
+                if (cudaError_t e = cudaMemcpyAsync(bins + at, s.bins2 + p2.bin_off[b],
+                                                    sizeof(int32_t) * size_t(rows),
+                                                    cudaMemcpyDeviceToDevice, stream);
+                    e != cudaSuccess)
+                    return bail(cuda_fail(e, "copy fill bins"));
+            p2.bin_off[b] = at;
+            at += rows;
+        }
         if (pa.bitmaps != nullptr) {
             void* bm = nullptr;
             B200_STEP(plan_alloc(plan, &bm, sizeof(uint32_t) * size_t(pa.words) * size_t(pa.nmaps),
@@ -1639,16 +1778,24 @@ spgemm_status transpose(spgemm_handle_s* h, const spgemm_csr_view* A, spgemm_csr
     }));
     const Ladder lad = make_ladder(tl, ntl, h->min_tr_bin);
     const int nctas = bin_ctas(n);
-    B200_STEP(timed(h, "tr_hist", 2, -1, n, stream, [&](cudaStream_t ss) {
-        return launch_nnz_hist(T->rpt, n, s.hist2, s.cta_sum, s.plan2, lad, ss);
-    }));
-    B200_STEP(timed(h, "tr_offsets", 2, -1, n, stream, [&](cudaStream_t ss) {
-        return launch_bin_offsets(s.hist2, nctas, s.cta_sum, s.plan2, lad, ss);
-    }));
-    B200_STEP(timed(h, "tr_scan_scatter", 2, -1, n, stream, [&](cudaStream_t ss) {
-        return launch_bin_scatter(T->rpt, n, s.hist2, s.cta_sum, s.bins2, s.plan2, lad, true,
-                                  ss);
-    }));
+    const bool append = n <= kAppendMaxRows;
+    if (append) {
+        B200_STEP(timed(h, "tr_scan_bins", 2, -1, n, stream, [&](cudaStream_t ss) {
+            return launch_rpt_scan_append(T->rpt, n, s.scan_state, s.plan2, s.status, s.bins2, n,
+                                          lad, ss);
+        }));
+    } else {
+        B200_STEP(timed(h, "tr_hist", 2, -1, n, stream, [&](cudaStream_t ss) {
+            return launch_nnz_hist(T->rpt, n, s.hist2, s.cta_sum, s.plan2, lad, ss);
+        }));
+        B200_STEP(timed(h, "tr_offsets", 2, -1, n, stream, [&](cudaStream_t ss) {
+            return launch_bin_offsets(s.hist2, nctas, s.cta_sum, s.plan2, lad, ss);
+        }));
+        B200_STEP(timed(h, "tr_scan_scatter", 2, -1, n, stream, [&](cudaStream_t ss) {
+            return launch_bin_scatter(T->rpt, n, s.hist2, s.cta_sum, s.bins2, s.plan2, lad, true,
+                                      ss);
+        }));
+    }
     B200_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&keys),
                                       kTrRecBytes * size_t(nnz), h->pool, stream),
               "allocate transpose records");
@@ -1661,7 +1808,8 @@ spgemm_status transpose(spgemm_handle_s* h, const spgemm_csr_view* A, spgemm_csr
     T->nnz = nnz;
     B200_STEP(sync_mirror(h, stream, s.plan2, s));
     B200_STEP(status_to_error(h->mirror->status));
-    const Plan plan = h->mirror->plan;
+    Plan plan = h->mirror->plan;
+    if (append) list_offsets(&plan, ntl, n);
     if (plan.total_key != nnz)
         return bail(fail(SPGEMM_ERR_INVALID_ARG, "A.col holds a column index outside [0, A.n)"));
     h->info.nnz = nnz;
