@@ -16,6 +16,7 @@
 #include <cooperative_groups.h>
 
 #include "cta.cuh"
+#include "fill.cuh"
 #include "kernels.hpp"
 #include "sort.cuh"
 
@@ -24,16 +25,6 @@ namespace cg = cooperative_groups;
 namespace b200 {
 
 namespace {
-
-template<typename V>
-__device__ __forceinline__ V ldv(const void* base, int i) {
-    return __ldg(static_cast<const V*>(base) + i);
-}
-
-// Entries of a row's slot at c0: its exact nnz, or in one-pass mode its NIP.
-__device__ __forceinline__ int slot_entries(const ProductArgs& p, int row, int c0) {
-    return p.row_slot != nullptr ? p.row_slot[row] : p.c_rpt[row + 1] - c0;
-}
 
 // A row of C whose A row holds ONE entry (a_ik at column k) is a_ik times B's
 // row k: its columns are B's (sorted, duplicate-free) and each value is one
@@ -152,8 +143,6 @@ __global__ __launch_bounds__(THREADS) void k_s2n_team(ProductArgs p) {
 // and no atomics, and sums each entry of C in the oracle's (Gustavson) order.
 // The keys need B.n <= 2^(31 - SHIFT); the ladder that holds these kernels is
 // used only for B.n <= kBitmapCols = 2^20 (SHIFT <= 10).
-constexpr int ilog2(int x) { return x <= 1 ? 0 : 1 + ilog2(x >> 1); }
-
 template<typename V, int G, int THREADS, int NMAX>
 struct EscLayout {
     static constexpr int T = next_pow2(NMAX);  // sort capacity of a team
@@ -596,24 +585,30 @@ __global__ __launch_bounds__(THREADS) void k_esc_cta(ProductArgs p) {
 }
 
 // Compression of the team bins, sampled: `samples` rows spread evenly over
-// A are counted exactly over their first kSampleProducts products (one warp
-// per row, a 1024-slot shared hash set) when their NIP is at most the last
-// team bin's limit, and those products and their distinct columns are summed
-// per team bin (binned by NIP with the ladder's limits); the NIP of every
-// sampled row, and of the longer ones apart, is summed too.  It needs A and B only, so it runs
-// on a side stream beside the NIP pass; the host reads the sums with the NIP
-// plan.  They choose one pass or two (rows above the team bins that repeat
-// many columns fill small nnz-sized tables only in two passes) and let a
-// team bin expand-sort-compress only when its rows repeat few columns: ESC
-// sorts every product, the hash bins only the distinct columns.
+// A, one warp per row with a 1024-slot shared hash set.  Rows up to the last
+// team bin's limit: their first kSampleProducts products and distinct columns
+// are counted exactly and summed per team bin (binned by NIP with the ladder's
+// limits).  A row that already repeats columns there is walked on, to
+// kSampleMore products, and these sums (all_*) join the first ones of the rows
+// that do not; rows past the last team bin, up to kSampleMaxNip products, join
+// the all_* sums only, as a class of their own.  The NIP of every sampled row,
+// of the longer ones apart, and the rows' widest column spans are kept too.
+// It needs A and B only, so it runs on a side stream beside the NIP pass; the
+// host reads the sums with the NIP plan.  They choose one pass or two (rows
+// above the team bins that repeat many columns fill small nnz-sized tables only
+// in two passes), let a team bin expand-sort-compress only when its rows repeat
+// few columns (ESC sorts every product, the hash bins only the distinct
+// columns), and size the column-window bins' bitmaps and sums.
 constexpr int kSampleWarps = 8;
 constexpr int kSampleSlots = 1024;
-constexpr int kSampleProducts = 256;  // products counted per sampled row
+constexpr int kSampleProducts = 256;
+constexpr int kSampleMore = 3 * kSampleSlots / 4;
 
 __global__ __launch_bounds__(kSampleWarps * kWarp) void k_esc_sample(ProductArgs p, int32_t m,
                                                                       int32_t samples,
                                                                       EscLimits lim,
                                                                       EscSample* out) {
+    constexpr unsigned kFull = 0xffffffffu;
     __shared__ int32_t s_tab[kSampleWarps][kSampleSlots];
     const int lane = threadIdx.x & 31;
     const int wid = threadIdx.x >> 5;
@@ -623,35 +618,57 @@ __global__ __launch_bounds__(kSampleWarps * kWarp) void k_esc_sample(ProductArgs
     const int a0 = p.a_rpt[row];
     const int a1 = p.a_rpt[row + 1];
     const int cap = lim.limit[kEscBins - 1];
+    auto add = [&](int64_t* to, int64_t v) {
+        atomicAdd(reinterpret_cast<unsigned long long*>(to), static_cast<unsigned long long>(v));
+    };
     auto count_nip = [&](int64_t v, bool above) {
         if (lane == 0) {
-            atomicAdd(reinterpret_cast<unsigned long long*>(&out->nip_seen),
-                      static_cast<unsigned long long>(v));
-            if (above)
-                atomicAdd(reinterpret_cast<unsigned long long*>(&out->nip_above),
-                          static_cast<unsigned long long>(v));
+            add(&out->nip_seen, v);
+            if (above) add(&out->nip_above, v);
         }
     };
     if (a1 - a0 > cap) {  // more products than the team bins take (>= a1 - a0)
         count_nip(a1 - a0, true);
         return;
     }
-    int nip = 0;
+    long long nip_ll = 0;
+    int lo = INT32_MAX;
+    int hi = -1;
     for (int e = a0 + lane; e < a1; e += kWarp) {
         const int c = __ldg(p.a_col + e);
-        nip += __ldg(p.b_rpt + c + 1) - __ldg(p.b_rpt + c);
+        const int s0 = __ldg(p.b_rpt + c);
+        const int s1 = __ldg(p.b_rpt + c + 1);
+        nip_ll += s1 - s0;
+        if (s0 < s1) {
+            lo = min(lo, __ldg(p.b_col + s0));
+            hi = max(hi, __ldg(p.b_col + s1 - 1));
+        }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) nip += __shfl_xor_sync(0xffffffffu, nip, o);
-    if (nip == 0) return;
-    count_nip(nip, nip > cap);
-    if (nip > cap || nip > 3 * kSampleSlots / 4) return;
+    for (int o = 16; o > 0; o >>= 1) nip_ll += __shfl_xor_sync(kFull, nip_ll, o);
+    if (nip_ll == 0) return;
+    count_nip(nip_ll, nip_ll > cap);
+    if (nip_ll > kSampleMaxNip) return;
+    const int nip = static_cast<int>(nip_ll);
+    lo = __reduce_min_sync(kFull, lo);
+    hi = __reduce_max_sync(kFull, hi);
     int b = 0;
-    while (nip > lim.limit[b]) b++;
-    // count the row's first kSampleProducts products only (the walk's latency
-    // is the sample's cost): the A entries up to the one that reaches them
-    int a_cut = a1;
-    if (nip > kSampleProducts) {
+    while (b < kEscBins && nip > lim.limit[b]) b++;
+    int32_t* tab = s_tab[wid];
+    for (int i = lane; i < kSampleSlots; i += kWarp) tab[i] = kEmpty;
+    __syncwarp();
+    int fresh = 0;
+    // the A entries [from, to): their first `most` products past `done`
+    auto insert = [&](int from, int to, int done, int most) {
+        team_for_products_at<kWarp>(p.a_col, p.b_rpt, from, to, [&](int qb, int, int q) {
+            if (done + q < most)
+                fresh += table_insert(tab, kSampleSlots, __ldg(p.b_col + qb), p.status, row);
+        });
+        return __reduce_add_sync(kFull, fresh);
+    };
+    // the entries that hold the first `most` products: [a0, cut), and the
+    // products in them
+    auto cut_at = [&](int most, int& products) {
         int run = 0;
         for (int base = a0; base < a1; base += kWarp) {
             const int e = base + lane;
@@ -660,32 +677,43 @@ __global__ __launch_bounds__(kSampleWarps * kWarp) void k_esc_sample(ProductArgs
                 const int c = __ldg(p.a_col + e);
                 len = __ldg(p.b_rpt + c + 1) - __ldg(p.b_rpt + c);
             }
-            const int inc = team_inclusive_scan<kWarp>(0xffffffffu, len, lane);
-            const unsigned hit = __ballot_sync(0xffffffffu, run + inc >= kSampleProducts);
+            const int inc = team_inclusive_scan<kWarp>(kFull, len, lane);
+            const unsigned hit = __ballot_sync(kFull, run + inc >= most);
             if (hit != 0u) {
-                a_cut = base + __ffs(hit);
-                break;
+                const int at = __ffs(hit) - 1;
+                products = run + __shfl_sync(kFull, inc, at);
+                return base + at + 1;
             }
-            run += __shfl_sync(0xffffffffu, inc, kWarp - 1);
+            run += __shfl_sync(kFull, inc, kWarp - 1);
         }
+        products = run;
+        return a1;
+    };
+    int seen = nip;
+    const int cut = nip > kSampleProducts ? cut_at(kSampleProducts, seen) : a1;
+    const int first_nip = min(nip, kSampleProducts);
+    const int first = insert(a0, cut, 0, kSampleProducts);
+    int all_nip = first_nip;
+    int all = first;
+    // repeats in the first products: walk on (whole B rows; the table holds
+    // kSampleMore columns at most)
+    if (nip > kSampleProducts && 4 * first_nip >= 5 * first) {
+        int done = seen;
+        const int cut2 = nip > kSampleMore ? cut_at(kSampleMore, done) : a1;
+        // (the cut row's products past kSampleProducts were skipped above)
+        all = insert(cut, cut2, seen, kSampleMore);
+        all_nip = min(nip, kSampleMore) - (seen - kSampleProducts);
     }
-    int32_t* tab = s_tab[wid];
-    for (int i = lane; i < kSampleSlots; i += kWarp) tab[i] = kEmpty;
-    __syncwarp();
-    team_for_products_at<kWarp>(p.a_col, p.b_rpt, a0, a_cut, [&](int qb, int, int q) {
-        if (q < kSampleProducts)
-            table_insert(tab, kSampleSlots, __ldg(p.b_col + qb), p.status, row);
-    });
-    __syncwarp();
-    int cnt = 0;
-    for (int i = lane; i < kSampleSlots; i += kWarp) cnt += tab[i] != kEmpty;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     if (lane == 0) {
-        atomicAdd(reinterpret_cast<unsigned long long*>(&out->nip[b]),
-                  static_cast<unsigned long long>(min(nip, kSampleProducts)));
-        atomicAdd(reinterpret_cast<unsigned long long*>(&out->nnz[b]),
-                  static_cast<unsigned long long>(cnt));
+        if (b < kEscBins) {
+            add(&out->nip[b], first_nip);
+            add(&out->nnz[b], first);
+        }
+        add(&out->all_nip[b], all_nip);
+        add(&out->all_nnz[b], all);
+        add(&out->row_nip[b], nip);
+        add(&out->rows[b], 1);
+        if (hi >= lo) atomicMax(&out->span[b], hi - lo + 1);
     }
 }
 
@@ -699,12 +727,11 @@ struct CtaLayout {
 };
 
 template<typename V, int THREADS, int T, int CAP>
-__global__ __launch_bounds__(THREADS) void k_s2n_cta(ProductArgs p) {
+__device__ __forceinline__ void s2n_cta_row(const ProductArgs& p, int row) {
     using L = CtaLayout<THREADS, T, CAP>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     int32_t* keys = reinterpret_cast<int32_t*>(smem_raw);
     auto& sc = *reinterpret_cast<CtaScratch<THREADS>*>(smem_raw + L::keys_bytes);
-    const int row = p.rows[blockIdx.x];
     const int c0 = p.c_rpt[row];
     // the row's exact nnz, or in one-pass mode its NIP (an upper bound)
     const int bound = slot_entries(p, row, c0);
@@ -743,6 +770,21 @@ __global__ __launch_bounds__(THREADS) void k_s2n_cta(ProductArgs p) {
         const int pos = lower_bound_present_swz(keys, nnz, key);
         atomicAdd(out + pos, ldv<V>(p.a_val, ai) * ldv<V>(p.b_val, qb));
     });
+}
+
+template<typename V, int THREADS, int T, int CAP>
+__global__ __launch_bounds__(THREADS) void k_s2n_cta(ProductArgs p) {
+    s2n_cta_row<V, THREADS, T, CAP>(p, p.rows[blockIdx.x]);
+}
+
+// The column-window bins' fail list (its length is on the device): a fixed grid.
+template<typename V, int THREADS, int T, int CAP>
+__global__ __launch_bounds__(THREADS) void k_s2n_cta_spill(ProductArgs p) {
+    const int nrows = *p.win_count;
+    for (int rid = blockIdx.x; rid < nrows; rid += gridDim.x) {
+        s2n_cta_row<V, THREADS, T, CAP>(p, p.win_rows[rid]);
+        __syncthreads();
+    }
 }
 
 // Bitmap bin (B.n <= kBitmapCols): the row's hash table is the identity hash
@@ -1157,6 +1199,13 @@ cudaError_t launch_esc_cta_split(const ProductArgs& p, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+template<typename V>
+cudaError_t launch_win_spill(const ProductArgs& p, cudaStream_t s) {
+    const int sms = p.sm_count > 0 ? p.sm_count : 148;
+    k_s2n_cta_spill<V, 256, 4096, 3072><<<2 * sms, 256, CtaLayout<256, 4096, 3072>::bytes, s>>>(p);
+    return cudaGetLastError();
+}
+
 template<typename V, int THREADS, int T, int CAP>
 cudaError_t launch_cta(const ProductArgs& p, cudaStream_t s) {
     k_s2n_cta<V, THREADS, T, CAP>
@@ -1409,6 +1458,7 @@ cudaError_t prepare_one() {
     B200_SMEM((k_s2n_team<V, 16, 256, 256>), (team_smem<16, 256, 256>()));
     B200_SMEM((k_s2n_team<V, 32, 256, 1024>), (team_smem<32, 256, 1024>()));
     B200_SMEM((k_s2n_cta<V, 256, 4096, 3072>), (CtaLayout<256, 4096, 3072>::bytes));
+    B200_SMEM((k_s2n_cta_spill<V, 256, 4096, 3072>), (CtaLayout<256, 4096, 3072>::bytes));
     B200_SMEM((k_s2n_cta<V, 512, 16384, 12288>), (CtaLayout<512, 16384, 12288>::bytes));
     B200_SMEM((k_s2n_cta<V, 1024, 43008, 32768>), (CtaLayout<1024, 43008, 32768>::bytes));
     B200_SMEM((k_s2n_bitmap<V, 1024, kBitmapCols>), (BitmapLayout<V, 1024, kBitmapCols>::bytes));
@@ -1424,6 +1474,14 @@ cudaError_t prepare_one() {
 }
 
 }  // namespace
+
+cudaError_t launch_win_spill_f64(const ProductArgs& p, cudaStream_t s) {
+    return launch_win_spill<double>(p, s);
+}
+
+cudaError_t launch_win_spill_f32(const ProductArgs& p, cudaStream_t s) {
+    return launch_win_spill<float>(p, s);
+}
 
 int s2n_ladder_f64(const BinLauncher** out) {
     *out = S2nLadder<double>::entries;

@@ -47,10 +47,9 @@ __global__ __launch_bounds__(THREADS) void k_sym1_team(ProductArgs p) {
 }
 
 template<int THREADS, int T>
-__global__ __launch_bounds__(THREADS) void k_sym1_cta(ProductArgs p) {
+__device__ __forceinline__ void sym1_cta_row(const ProductArgs& p, int row) {
     extern __shared__ int32_t smem[];
     auto& sc = *reinterpret_cast<CtaScratch<THREADS>*>(smem + T);
-    const int row = p.rows[blockIdx.x];
     for (int i = threadIdx.x; i < T; i += THREADS) smem[i] = kEmpty;
     __syncthreads();
     const int a0 = p.a_rpt[row];
@@ -61,6 +60,21 @@ __global__ __launch_bounds__(THREADS) void k_sym1_cta(ProductArgs p) {
     });
     cnt = block_sum<THREADS>(cnt, sc.warp_tot);
     if (threadIdx.x == 0) p.c_rpt[row] = cnt;
+}
+
+template<int THREADS, int T>
+__global__ __launch_bounds__(THREADS) void k_sym1_cta(ProductArgs p) {
+    sym1_cta_row<THREADS, T>(p, p.rows[blockIdx.x]);
+}
+
+// The column-window bins' fail list (its length is on the device): a fixed grid.
+template<int THREADS, int T>
+__global__ __launch_bounds__(THREADS) void k_sym1_cta_spill(ProductArgs p) {
+    const int nrows = *p.win_count;
+    for (int rid = blockIdx.x; rid < nrows; rid += gridDim.x) {
+        sym1_cta_row<THREADS, T>(p, p.win_rows[rid]);
+        __syncthreads();
+    }
 }
 
 // Cluster bin: the row's table is split over the cluster's CTAs; slot h of the
@@ -281,6 +295,12 @@ const BinLauncher kLadder[] = {
 
 }  // namespace
 
+cudaError_t launch_win_spill_count(const ProductArgs& p, cudaStream_t s) {
+    const int sms = p.sm_count > 0 ? p.sm_count : 148;
+    k_sym1_cta_spill<256, kC4><<<2 * sms, 256, kLadder[4].smem, s>>>(p);
+    return cudaGetLastError();
+}
+
 int sym1_ladder(const BinLauncher** out) {
     *out = kLadder;
     return static_cast<int>(sizeof(kLadder) / sizeof(kLadder[0]));
@@ -297,6 +317,7 @@ cudaError_t sym1_prepare() {
     B200_SMEM((k_sym1_team<16, 256, kT2>), kLadder[2].smem);
     B200_SMEM((k_sym1_team<32, 256, kT3>), kLadder[3].smem);
     B200_SMEM((k_sym1_cta<256, kC4>), kLadder[4].smem);
+    B200_SMEM((k_sym1_cta_spill<256, kC4>), kLadder[4].smem);
     B200_SMEM((k_sym1_cta<512, kC5>), kLadder[5].smem);
     B200_SMEM((k_sym1_cta<1024, kC6>), kLadder[6].smem);
     B200_SMEM((k_sym1_cluster<1024, kC6>), kLadder[7].smem);

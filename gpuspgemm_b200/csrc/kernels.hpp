@@ -66,6 +66,12 @@ struct ProductArgs {
     // in row order (nullptr: c_rpt[row + 1] - c_rpt[row]).  It may be row_nnz
     // itself: a row is read and then written by the one kernel that fills it.
     const int32_t* row_slot;
+    // column-window bins: the bitmap's words and the sums of a row, and the
+    // list of the rows that did not fit (launch_win_spill*)
+    int32_t win_words;
+    int32_t win_cap;
+    int32_t* win_rows;
+    int32_t* win_count;
     // SMs of the device (persistent kernels size their grid by it; 0: 148)
     int32_t sm_count;
     // persistent bins: a device counter the CTAs take their next row from
@@ -83,6 +89,8 @@ struct BinLauncher {
     size_t smem;            // dynamic shared memory per CTA
     const char* name;
     cudaError_t (*launch)(const ProductArgs&, cudaStream_t);
+    int32_t win_words;      // column-window bins (ProductArgs' fields)
+    int32_t win_cap;
 };
 
 // One-pass fill (no count phase) when its temporaries, NIP entries of column
@@ -120,6 +128,24 @@ constexpr int kEscCtaSmall = 1024;
 const BinLauncher* s2n_esc_cta_f64(int which);
 const BinLauncher* s2n_esc_cta_f32(int which);
 
+// Column-window bins (k_win.cu): rows whose columns lie inside `words` * 32
+// columns of B, with at most `cap` distinct ones, a team of `lanes` lanes each.
+constexpr int kWinMaxWords = 2048;
+BinLauncher win_fill_bin(int value_bytes, int lanes, int words, int cap);
+BinLauncher win_count_bin(int lanes, int words);
+// A thread per row of at most kThreadCap columns (others join the same list),
+// for at least kThreadRows rows and B.n <= kThreadCols.
+constexpr int kThreadCap = 16;
+constexpr int kThreadRows = 1 << 16;
+constexpr int32_t kThreadCols = int32_t(1) << 26;
+BinLauncher thread_fill_bin(int value_bytes);
+cudaError_t win_prepare();
+// The rows that did not fit (their number is on the device), by hashing: counts
+// of rows of up to 3,072 products, fills of rows of up to 3,072 entries.
+cudaError_t launch_win_spill_count(const ProductArgs& p, cudaStream_t s);
+cudaError_t launch_win_spill_f64(const ProductArgs& p, cudaStream_t s);
+cudaError_t launch_win_spill_f32(const ProductArgs& p, cudaStream_t s);
+
 // Sampled compression of the first kEscBins fill bins of a one-pass product:
 // the NIP and exact nnz of up to `samples` rows spread evenly over A, summed
 // per team bin (rows binned by NIP with `lim`; rows above the last limit are
@@ -156,7 +182,17 @@ struct EscSample {
     int64_t nip_above;  // longer than the last limit), and of those above it
     int32_t split;      // written by launch_esc_decide
     int32_t pad;
+    // the same sums over more of the rows' products (see k_esc_sample), the
+    // sampled rows and their widest column span, with one class more: rows
+    // past the last team bin, up to kSampleMaxNip products
+    int64_t all_nip[kEscBins + 1];
+    int64_t all_nnz[kEscBins + 1];
+    int64_t row_nip[kEscBins + 1];
+    int64_t rows[kEscBins + 1];
+    int32_t span[kEscBins + 1];
+    int32_t pad2;
 };
+constexpr int kSampleMaxNip = 3072;
 cudaError_t launch_esc_sample(const ProductArgs& p, int32_t m, int32_t samples,
                               const EscLimits& lim, EscSample* out, cudaStream_t s);
 // The fill binning's limits, decided on the device from the sample: when the

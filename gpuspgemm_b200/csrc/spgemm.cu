@@ -15,6 +15,7 @@
 // cleanup.cuh:15-31); here streams, events and scratch live in the handle.
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -69,6 +70,8 @@ struct Scratch {
     int32_t* bins2;
     int32_t* fail_rows;
     int32_t* fail_count;
+    int32_t* win_rows;   // rows that did not fit a column-window bin
+    int32_t* win_count;
     EscSample* sample;
     Ladder* dladder;  // the one-pass fill binning's limits, decided on the device
     int32_t* work;    // one row counter per fill bin (persistent bins)
@@ -194,6 +197,7 @@ spgemm_status ensure_scratch(spgemm_handle_s* h, int32_t m, Scratch* s, cudaStre
     const size_t o_plan1 = take(sizeof(Plan));
     const size_t o_plan2 = take(sizeof(Plan));
     const size_t o_fail_count = take(sizeof(int32_t));
+    const size_t o_win_count = take(sizeof(int32_t));
     const size_t o_sample = take(sizeof(EscSample));
     const size_t o_dladder = take(sizeof(Ladder));
     const size_t o_scan = take(sizeof(unsigned long long) * (1 + kScanMaxTiles));
@@ -207,6 +211,7 @@ spgemm_status ensure_scratch(spgemm_handle_s* h, int32_t m, Scratch* s, cudaStre
     const size_t o_bins1 = take(sizeof(int32_t) * mm * (append ? kListBins : 1));
     const size_t o_bins2 = append ? o_bins1 : take(sizeof(int32_t) * mm);
     const size_t o_fail = take(sizeof(int32_t) * mm);
+    const size_t o_win = take(sizeof(int32_t) * mm);
     const size_t o_work = take(sizeof(int32_t) * kMaxBins);
     if (spgemm_status st = regrow(h, &h->scratch, &h->scratch_bytes, off + off / 4, stream);
         st != SPGEMM_OK)
@@ -225,6 +230,8 @@ spgemm_status ensure_scratch(spgemm_handle_s* h, int32_t m, Scratch* s, cudaStre
     s->bins1 = reinterpret_cast<int32_t*>(b + o_bins1);
     s->bins2 = reinterpret_cast<int32_t*>(b + o_bins2);
     s->fail_rows = reinterpret_cast<int32_t*>(b + o_fail);
+    s->win_rows = reinterpret_cast<int32_t*>(b + o_win);
+    s->win_count = reinterpret_cast<int32_t*>(b + o_win_count);
     s->work = reinterpret_cast<int32_t*>(b + o_work);
     s->scan_state = reinterpret_cast<unsigned long long*>(b + o_scan);
     return SPGEMM_OK;
@@ -447,6 +454,8 @@ spgemm_status launch_bins(spgemm_handle_s* h, const BinLauncher* bins, int nb, i
         ProductArgs a = base;
         a.rows = row_lists + plan.bin_off[b];
         a.nrows = rows;
+        a.win_words = bins[b].win_words;
+        a.win_cap = bins[b].win_cap;
         a.work = base.work != nullptr ? base.work + b : nullptr;
         cudaStream_t s = nside == 0 ? main
                                     : h->side[next == 0 || nside == 1 ? 0 : 1 + (next - 1) % (nside - 1)];
@@ -512,6 +521,47 @@ ListLadder list_ladder(const Ladder& fill, bool esc) {
     }
     l.lad.nb = nb;
     return l;
+}
+
+// Column-window bins take a bin's rows when the sampled rows (two passes: the
+// product) repeat their columns at least kWinMinRatio times -- their walks then
+// cost less than the hash bins' and than sorting every product -- and the
+// sampled span needs at most kWinMaxWords words and kWinWordsPerNip words per
+// product of a row (the bitmap is cleared and scanned whole).
+constexpr double kWinMinRatio = 1.5;
+constexpr double kWinWordsPerNip = 4.0;
+// A thread per row (rows of at most kThreadCap columns) from this ratio on.
+constexpr double kThreadMinRatio = 3.0;
+// What a row may have past the sampled rows' span and past its columns as the
+// sampled ratio estimates them; rows past that go to the fail list.
+constexpr double kWinSpanSpare = 1.1;
+constexpr double kWinColumnSpare = 1.3;
+
+// Lanes per row for B rows of this mean length.
+int win_lanes(double mean) {
+    int g = 4;
+    while (g < 32 && g < mean) g *= 2;
+    return g;
+}
+
+// The bitmap's words for the sampled classes [first, last], or 0 when they do
+// not suit the window bins.
+int win_words(const EscSample& es, int first, int last) {
+    int64_t nip = 0, nnz = 0, row_nip = 0, rows = 0;
+    int32_t span = 0;
+    for (int b = first; b <= last; b++) {
+        nip += es.all_nip[b];
+        nnz += es.all_nnz[b];
+        row_nip += es.row_nip[b];
+        rows += es.rows[b];
+        span = std::max(span, es.span[b]);
+    }
+    if (rows <= 0 || static_cast<double>(nip) < kWinMinRatio * static_cast<double>(nnz)) return 0;
+    const double words = std::ceil(kWinSpanSpare * span / 32.0) + 1.0;
+    if (words > kWinMaxWords ||
+        words > kWinWordsPerNip * static_cast<double>(row_nip) / static_cast<double>(rows))
+        return 0;
+    return static_cast<int>(words);
 }
 
 Ladder scaled_ladder(const BinLauncher* bins, int nb, int min_bin, double team_scale,
@@ -643,8 +693,8 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     // or two and, per fill bin, expand-sort-compress or hashing.
     const Ladder ladf = make_ladder(fil, nfil, h->min_num_bin);
     const int esc_mode = (narrow && h->esc != 2) ? h->esc : 2;
-    const bool sampled = cr == nullptr && h->one_pass != 2 && A->nnz >= kSampleMinNnz &&
-                         (h->one_pass == 0 || esc_mode == 0);
+    const bool sampled = A->nnz >= kSampleMinNnz &&
+                         (h->esc != 2 || (cr == nullptr && h->one_pass == 0));
     if (sampled) {
         EscLimits el{};
         for (int b = 0; b < kEscBins; b++) el.limit[b] = fil[b].limit;
@@ -799,12 +849,16 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     } else {
         B200_STEP(count_binning());
     }
+    if (sampled && !early)
+        if (cudaError_t e = cudaStreamWaitEvent(stream, h->ev_sample, 0); e != cudaSuccess)
+            return bail(cuda_fail(e, "join the sample stream"));
     mark(0);
     if (mirror_pending) {
-        B200_STEP(mirror_finish(h, s.plan1, s, early && sampled, early ? fill_plan : nullptr));
+        B200_STEP(mirror_finish(h, s.plan1, s, sampled, early ? fill_plan : nullptr));
     } else {
-        B200_STEP(sync_mirror(h, stream, s.plan1, s, early && sampled, early ? fill_plan : nullptr));
+        B200_STEP(sync_mirror(h, stream, s.plan1, s, sampled, early ? fill_plan : nullptr));
     }
+    const EscSample es = h->mirror->sample;  // read when `sampled`
     mark(1);
     B200_STEP(status_to_error(h->mirror->status));
     Plan p1 = h->mirror->plan;  // bin sizes valid once the count binning ran
@@ -828,6 +882,8 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     pa.cluster = h->cluster;
     pa.fail_rows = s.fail_rows;
     pa.fail_count = s.fail_count;
+    pa.win_rows = s.win_rows;
+    pa.win_count = s.win_count;
     pa.words = (static_cast<int64_t>(n) + 31) / 32;
     pa.sm_count = h->sm_count;
     pa.work = s.work;
@@ -885,7 +941,6 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
         mark(3);
         B200_ONE(status_to_error(h->mirror->status));
         Plan pf = h->mirror->plan_b;
-        const EscSample es = h->mirror->sample;
         if (append) list_offsets(&pf, lists.lad.nb, m);
         // sampled: the NIP of rows above the team bins, the team bins' NIP/nnz
         int64_t team_nip = 0;
@@ -946,6 +1001,34 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
                 }
             }
         }
+        // the fill bins' rows (append binning counts by finer lists)
+        int32_t bin_rows[kMaxBins] = {};
+        for (int e = 0; e < (append ? lists.lad.nb : nfil); e++)
+            bin_rows[append ? lists.fill_bin(e, split) : e] += pf.bin_size[e];
+        // column-window bins where the sampled rows repeat their columns
+        bool windows = false;
+        if (sampled && h->esc != 2) {
+            const int lanes = win_lanes(static_cast<double>(nip_total) / A->nnz);
+            for (int b = 0; b <= kEscBins; b++) {
+                if ((h->info.esc_mask >> b) & 1) continue;
+                if (es.all_nnz[b] <= 0) continue;
+                const int most = std::min(fil[b].limit, p1.max_key);
+                const double ratio = static_cast<double>(es.all_nip[b]) /
+                                     static_cast<double>(es.all_nnz[b]);
+                const int columns =
+                    std::min(most, static_cast<int>(kWinColumnSpare * most / ratio) + 2);
+                if (ratio >= kThreadMinRatio && columns <= kThreadCap && n <= kThreadCols &&
+                    bin_rows[b] >= kThreadRows) {
+                    one_fil[b] = thread_fill_bin(sizeof(V));
+                    windows = true;
+                    continue;
+                }
+                const int words = win_words(es, b, b);
+                if (words == 0) continue;
+                one_fil[b] = win_fill_bin(sizeof(V), lanes, words, columns);
+                windows = true;
+            }
+        }
         // append binning: the kernel of each list
         BinLauncher list_fil[kMaxBins];
         int list_ids[kMaxBins];
@@ -981,6 +1064,10 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
         mark(4);
         B200_ONE(launch_bins(h, fill_bins, nfill, 3, pf, s.bins2, pa, stream,
                              append ? list_ids : nullptr));
+        if (windows)
+            B200_ONE(timed(h, "win_spills", 3, -1, -1, stream, [&](cudaStream_t ss) {
+                return sizeof(V) == 8 ? launch_win_spill_f64(pa, ss) : launch_win_spill_f32(pa, ss);
+            }));
         // row pointer from the counts, into the plan the fill bins do not use
         // (reset if a pass has written it: its max and overflow only ever
         // grow): one look-back scan -- or, past its tile limit, a one-bin pass
@@ -1117,12 +1204,6 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
 #undef B200_ONE_CUDA
 #undef B200_ONE
     }
-    if (sampled && h->info.one_pass == 0) {
-        // two passes: the sample's work is not needed, but it still reads A
-        // and B; the final synchronisation must cover it
-        if (cudaError_t e = cudaStreamWaitEvent(stream, h->ev_sample, 0); e != cudaSuccess)
-            return bail(cuda_fail(e, "join the sample stream"));
-    }
     // the scan pass's plan: the one the fill binning by NIP used, if it ran
     Plan* const scan_plan = fill_plan;
     if (early || one_pass) {
@@ -1150,6 +1231,14 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     }
 
     // ---- sym1: exact nnz per row --------------------------------------------
+    // column-window bins for the team bins' rows where the sampled rows of all
+    // classes suit them
+    const int lanes = win_lanes(static_cast<double>(nip_total) / A->nnz);
+    const int windows = sampled && h->esc != 2 ? win_words(es, 0, kEscBins) : 0;
+    BinLauncher count_bins[kMaxBins];
+    for (int b = 0; b < nsym; b++)
+        count_bins[b] =
+            windows > 0 && sym[b].kind == BinKind::Team ? win_count_bin(lanes, windows) : sym[b];
     const int glob1 = nsym - 1;  // global bin (cluster spills, or the test knob)
     const int clus1 = nsym - 2;  // cluster bin
     const int32_t cluster_rows = p1.bin_size[clus1];
@@ -1200,12 +1289,22 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
             ProductArgs a = pa;
             a.rows = s.bins1 + p1.bin_off[b];
             a.nrows = rows;
-            B200_STEP(timed(h, sym[b].name, 1, b, rows, sym_side > 0 ? h->side[next] : stream,
-                            [&](cudaStream_t ss) { return sym[b].launch(a, ss); }));
+            a.win_words = count_bins[b].win_words;
+            B200_STEP(timed(h, count_bins[b].name, 1, b, rows,
+                            sym_side > 0 ? h->side[next] : stream,
+                            [&](cudaStream_t ss) { return count_bins[b].launch(a, ss); }));
             next = next + 1 < sym_side ? next + 1 : first;
         }
     }
     B200_STEP(join_streams(h, stream, sym_side));
+    if (windows > 0) {
+        B200_STEP(timed(h, "win_spills", 1, -1, -1, stream,
+                        [&](cudaStream_t ss) { return launch_win_spill_count(pa, ss); }));
+        // the fill's list starts empty
+        if (cudaError_t e = cudaMemsetAsync(s.win_count, 0, sizeof(int32_t), stream);
+            e != cudaSuccess)
+            return bail(cuda_fail(e, "reset the window bins' list"));
+    }
 
     // ---- scan pass: row pointer and fill bins -------------------------------
     const Ladder lad2 = scaled_ladder(fil, nfil, h->min_num_bin, cr ? cr->team_scale : 1.0,
@@ -1266,6 +1365,19 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
         pa.bitmaps = h->bitmaps;
         pa.nmaps = nmaps;
     }
+    // column-window bins, their sums sized by the rows' exact nnz
+    BinLauncher two_fil[kMaxBins];
+    for (int b = 0; b < nfil; b++) two_fil[b] = fil[b];
+    const double repeats = static_cast<double>(nip_total) / static_cast<double>(nnz);
+    const bool fill_windows = windows > 0 && repeats >= kWinMinRatio;
+    if (fill_windows)
+        for (int b = 0; b <= kEscBins; b++) {
+            const int cap = std::min(lad2.limit[b], p2.max_key);
+            two_fil[b] = repeats >= kThreadMinRatio && cap <= kThreadCap && n <= kThreadCols &&
+                                 p2.bin_size[b] >= kThreadRows
+                             ? thread_fill_bin(sizeof(V))
+                             : win_fill_bin(sizeof(V), lanes, windows, cap);
+        }
     mark(4);
     DevStatus* fill_status = s.status;
     if (cr != nullptr && cr->plan != nullptr) {
@@ -1297,15 +1409,29 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
         B200_STEP(plan_alloc(plan, reinterpret_cast<void**>(&work), sizeof(int32_t) * kMaxBins,
                              stream));
         pa.work = work;
+        if (fill_windows) {
+            void* list = nullptr;
+            B200_STEP(plan_alloc(plan, &list, sizeof(int32_t) * (size_t(m) + 1), stream));
+            pa.win_count = static_cast<int32_t*>(list);
+            pa.win_rows = pa.win_count + 1;
+        }
         pa.status = plan->status;
         fill_status = plan->status;
         const int saved_profile = h->profile;
         h->profile = 0;
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamBeginCapture(plan->capture, cudaStreamCaptureModeThreadLocal);
-        spgemm_status st = e == cudaSuccess
-                               ? launch_bins(h, fil, nfil, 3, p2, bins, pa, plan->capture)
-                               : cuda_fail(e, "begin capture");
+        spgemm_status st = e == cudaSuccess ? SPGEMM_OK : cuda_fail(e, "begin capture");
+        if (st == SPGEMM_OK && fill_windows) {
+            e = cudaMemsetAsync(pa.win_count, 0, sizeof(int32_t), plan->capture);
+            if (e != cudaSuccess) st = cuda_fail(e, "reset the window bins' list");
+        }
+        if (st == SPGEMM_OK) st = launch_bins(h, two_fil, nfil, 3, p2, bins, pa, plan->capture);
+        if (st == SPGEMM_OK && fill_windows) {
+            e = sizeof(V) == 8 ? launch_win_spill_f64(pa, plan->capture)
+                               : launch_win_spill_f32(pa, plan->capture);
+            if (e != cudaSuccess) st = cuda_fail(e, "window spills");
+        }
         const cudaError_t ee = cudaStreamEndCapture(plan->capture, &g);
         h->profile = saved_profile;
         if (st != SPGEMM_OK) {
@@ -1323,7 +1449,11 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
             cr->graph = g;
         }
     } else {
-        B200_STEP(launch_bins(h, fil, nfil, 3, p2, s.bins2, pa, stream));
+        B200_STEP(launch_bins(h, two_fil, nfil, 3, p2, s.bins2, pa, stream));
+        if (fill_windows)
+            B200_STEP(timed(h, "win_spills", 3, -1, -1, stream, [&](cudaStream_t ss) {
+                return sizeof(V) == 8 ? launch_win_spill_f64(pa, ss) : launch_win_spill_f32(pa, ss);
+            }));
     }
     mark(5);
     if (cudaError_t e = cudaMemcpyAsync(&h->mirror->status, fill_status, sizeof(DevStatus),
@@ -2191,6 +2321,7 @@ spgemm_status spgemm_create(spgemm_handle_t* handle, int device) {
     B200_TRY(cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, dev));
     B200_TRY(sym1_prepare());
     B200_TRY(s2n_prepare());
+    B200_TRY(win_prepare());
     B200_TRY(transpose_prepare());
     for (int i = 0; i < kMaxSide; i++) {
         // side stream 0 runs each phase's heaviest bin: the highest priority,
