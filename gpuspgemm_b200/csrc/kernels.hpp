@@ -95,10 +95,14 @@ struct BinLauncher {
 
 // One-pass fill (no count phase) when its temporaries, NIP entries of column
 // and value, fit this many bytes and the product has at least kOnePassMinNip
-// intermediate products (below that its extra host synchronisation and
-// launches cost more than the count phase it saves).
+// intermediate products, kOnePassMinNipUnsampled where the compression sample
+// did not run (its rows are then hashed, not sorted).  One pass against two,
+// whole calls, us: power-law FP64 30,000 rows at exponent 2.3 (NIP 192 k) 182
+// against 284, at 2.0 (839 k) 222 against 311; uniform 10,000 x 8 (640 k) 119
+// against 145; power-law 10,000 rows at 2.3 (66 k) 191 against 251.
 constexpr uint64_t kOnePassMaxBytes = uint64_t(4) << 30;
-constexpr int64_t kOnePassMinNip = int64_t(1) << 21;
+constexpr int64_t kOnePassMinNip = int64_t(1) << 16;
+constexpr int64_t kOnePassMinNipUnsampled = int64_t(1) << 21;
 // Symbolic count ladder (key = NIP of the row).
 int sym1_ladder(const BinLauncher** out);
 // Fused fill + sort + numeric ladder (key = nnz of the row), per value type.
@@ -160,12 +164,13 @@ constexpr double kEscMaxRatio[kEscBins] = {8.0, 8.0, 1.4, 1.1};
 // The one-pass ladder's bins that may expand-sort-compress: the team bins and
 // the 256-thread bin, which follows the sample of the largest team bin.
 constexpr int kEscLadderBins = kEscBins + 1;
-// The sample runs for products with at least this many entries in A.
-constexpr int64_t kSampleMinNnz = int64_t(1) << 16;
+// The sample runs for products with at least this many entries in A (a
+// smaller product's launches cost more than what it decides).
+constexpr int64_t kSampleMinNnz = (int64_t(1) << 15) + 1;
 // Products with at least this many entries in A are expected to run one pass:
 // they are binned for the fill right after the NIP pass, before the first
 // synchronisation (the count binning follows only if they run two).
-constexpr int64_t kEarlyOnePassNnz = int64_t(1) << 18;
+constexpr int64_t kEarlyOnePassNnz = kSampleMinNnz;
 // Auto mode keeps two passes when at least this share of the sampled NIP
 // lies in rows above the team bins (one pass bins them by NIP into the CTA
 // bins, two passes by nnz into small team tables) and the team bins' sampled

@@ -725,8 +725,11 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     // decided at the one synchronisation that follows; the count binning then
     // runs only if it turns out two-pass.  Its fill binning scans a copy of
     // the NIP per row, which the NIP pass writes beside C.rpt.
-    const bool early = cr == nullptr && h->one_pass != 2 &&
-                       (h->one_pass == 1 || A->nnz >= kEarlyOnePassNnz);
+    // (plans replay the two-pass fill; batches run one pass where their small
+    // rows may expand, sort and compress: 20 products, 32 M NIP, FP32, 1.86 -> 1.27 ms)
+    const bool may_one_pass =
+        h->one_pass != 2 && (cr == nullptr || (cr->plan == nullptr && narrow && h->esc != 2));
+    const bool early = may_one_pass && (h->one_pass == 1 || A->nnz >= kEarlyOnePassNnz);
     int32_t* off = nullptr;  // the one-pass NIP slots: a scan of the NIP per row
     bool off_written = false;
     if (early) {
@@ -902,9 +905,9 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     // repeat many columns); the binning by NIP is then the only work lost.
     const int64_t nip_total = p1.total_key;
     const bool one_pass =
-        cr == nullptr && h->one_pass != 2 && nip_total <= INT32_MAX &&
+        may_one_pass && nip_total <= INT32_MAX &&
         (h->one_pass == 1 ||
-         (nip_total >= kOnePassMinNip &&
+         (nip_total >= (sampled ? kOnePassMinNip : kOnePassMinNipUnsampled) &&
           static_cast<uint64_t>(nip_total) * (4 + sizeof(V)) <= kOnePassMaxBytes));
     h->info.one_pass = one_pass ? 1 : 0;
     if (one_pass) {
@@ -1603,9 +1606,8 @@ spgemm_status batch(spgemm_handle_s* h, const spgemm_batch_desc* d, const spgemm
         cr.cta_scale = cta_scale;
         cr.plan = plan;
         cr.launch_now = false;
-        // every group runs the two-pass path (a plan captures its fill; a plain
-        // batch measured no faster through the one-pass path, 4,096 products
-        // 472 vs 474 ms, and the served loop's batches slower)
+        // a plan's groups run the two-pass path (their fill is captured), a
+        // plain batch's the path that product() picks
         spgemm_status st = product<V>(h, &Ag, B, &Cg, stream, &cr);
         if (st != SPGEMM_OK) {
             h->checked = saved_checked;
