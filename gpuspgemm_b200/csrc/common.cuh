@@ -104,11 +104,12 @@ __device__ __forceinline__ void team_sync(unsigned mask) {
 // position of the B entry in B.col / B.val, a_index the position of the A
 // entry and q the product's place in the row's flattened sequence (products
 // of A entry a0 first, each B row in order).  All lanes of the team must call
-// this together (the shuffles are team-wide).
+// this together (the shuffles are team-wide).  With `most` given, only about
+// the first `most` products (whole steps of G).
 template<int G, typename F>
 __device__ __forceinline__ void team_for_products_at(const int32_t* __restrict__ a_col,
                                                      const int32_t* __restrict__ b_rpt, int a0,
-                                                     int a1, F&& f) {
+                                                     int a1, F&& f, int most = INT32_MAX) {
     const unsigned mask = team_mask<G>();
     const int lane = team_lane<G>();
     int off = 0;
@@ -124,7 +125,7 @@ __device__ __forceinline__ void team_for_products_at(const int32_t* __restrict__
         const int inc = team_inclusive_scan<G>(mask, len, lane);
         const int total = __shfl_sync(mask, inc, G - 1, G);
         const int exc = inc - len;
-        for (int q0 = 0; q0 < total; q0 += G) {
+        for (int q0 = 0; q0 < total && off + q0 < most; q0 += G) {
             const int q = q0 + lane;
             // largest source lane s with exc_s <= q (lanes with len 0 share exc
             // with their successor, so the result always has len_s > 0)

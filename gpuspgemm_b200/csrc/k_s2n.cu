@@ -141,8 +141,8 @@ __global__ __launch_bounds__(THREADS) void k_s2n_team(ProductArgs p) {
 // values in that order and writes the column and the sum to the next slot.
 // That needs no hash table, no second walk of the products, no binary search
 // and no atomics, and sums each entry of C in the oracle's (Gustavson) order.
-// The keys need B.n <= 2^(31 - SHIFT); the ladder that holds these kernels is
-// used only for B.n <= kBitmapCols = 2^20 (SHIFT <= 10).
+// The keys need B.n <= 2^(31 - SHIFT): kEscCols = 2^22 for the 512-product
+// kernel that one-pass products run.
 template<typename V, int G, int THREADS, int NMAX>
 struct EscLayout {
     static constexpr int T = next_pow2(NMAX);  // sort capacity of a team
@@ -240,7 +240,7 @@ __global__ __launch_bounds__(THREADS) void k_esc_team(ProductArgs p) {
 //      of the B-row lengths places each entry's first product;
 //   2. 32 products at a time, each lane finds its product's entry by a search
 //      over that scan, loads B's column and value, and stages the key (row in
-//      the batch << (20 + PB) | column << PB | product, PB = log2(32 K); the
+//      the batch << (22 + PB) | column << PB | product, PB = log2(32 K); the
 //      three fit 32 bits) and the product a_ik * b_kj in shared memory;
 //   3. a warp bitonic sort of the 32 K keys (element r * 32 + lane in
 //      register r of the lane) orders them by row, column and product; the
@@ -248,8 +248,7 @@ __global__ __launch_bounds__(THREADS) void k_esc_team(ProductArgs p) {
 //      (Gustavson's order, as the team kernels) and writes the column and sum
 //      at its rank in the row; the last element of each row writes the row's
 //      nnz.
-// Single-entry rows take the same path.  Needs B.n <= 2^20 (the ladder that
-// holds it) and the one-pass mode's NIP-sized slots; a row of more than 32 K
+// Single-entry rows take the same path.  Needs B.n <= kEscCols = 2^22 and the one-pass mode's NIP-sized slots; a row of more than 32 K
 // products is reported.  Per bin (1M power-law product, serialised): rows of
 // <= 12 products K = 1, 32 rows a warp (4-lane teams 0.092 -> 0.057 ms); <= 48
 // K = 2, 8 rows (8-lane teams 0.067 -> 0.060; 4 or 16 rows no better); <= 192
@@ -265,7 +264,8 @@ __global__ __launch_bounds__(THREADS) void k_esc_warp(ProductArgs p) {
     constexpr int NW = THREADS / kWarp;
     constexpr int CAP = kWarp * K;  // products per batch
     constexpr int PB = ilog2(CAP);  // bits of a product's place in the batch
-    constexpr int RS = 20 + PB;     // row-in-batch shift
+    constexpr int CB = ilog2(kEscCols);  // bits of a column
+    constexpr int RS = CB + PB;          // row-in-batch shift
     static_assert(RS + ilog2(2 * ROWS - 1) <= 32, "row, column and place fit 32 bits");
     constexpr unsigned kFull = 0xffffffffu;
     __shared__ uint32_t s_key[NW][CAP];
@@ -464,7 +464,7 @@ __global__ __launch_bounds__(THREADS) void k_esc_warp(ProductArgs p) {
                     if ((nk >> PB) != (kr >> PB)) break;
                     sum += vals[nk & (CAP - 1)];
                 }
-                p.c_col[out0 + rank - 1] = static_cast<int32_t>((kr >> PB) & 0xfffffu);
+                p.c_col[out0 + rank - 1] = static_cast<int32_t>((kr >> PB) & (kEscCols - 1));
                 static_cast<V*>(p.c_val)[out0 + rank - 1] = sum;
             }
             const uint32_t down = __shfl_down_sync(kFull, kr, 1);
@@ -485,28 +485,37 @@ __global__ __launch_bounds__(THREADS) void k_esc_warp(ProductArgs p) {
 // SHIFT)).  The keys are staged in product order and sorted by a stable
 // radix sort of their column bits only (sort.cuh cta_radix_sort: 3 passes
 // for B.n <= 2^21), so a column's products stay in product order.
+// With WIDE set, columns take more bits than a key has above its product number
+// (B.n > 2^(32 - SHIFT)): the bits above those, at most 7, wait in an array by
+// product number, and the radix sort takes one more pass on them.
 // Compression: each thread takes a contiguous run of sorted positions,
 // counts the column heads in it, a block scan gives its first output slot,
 // and each head sums its column's run (which may run into the next thread's
 // positions) in product order.
-template<typename V, int THREADS, int NMAX>
+template<typename V, int THREADS, int NMAX, bool WIDE = false>
 struct EscCtaLayout {
     static constexpr int P = next_pow2(NMAX);
     static constexpr int SHIFT = ilog2(P);
+    static constexpr int LOW = 32 - SHIFT;  // column bits in a key
+    static_assert(WIDE || LOW >= ilog2(kBitmapCols), "column bits");
+    static_assert(LOW + 7 >= ilog2(kEscCols), "column bits beside the key");
     static constexpr int RMAX = (NMAX + THREADS - 1) / THREADS;  // radix rounds per warp
     static constexpr size_t vals_bytes = sizeof(V) * NMAX;
     static constexpr size_t keys_bytes = sizeof(uint32_t) * NMAX;
     static constexpr size_t hist_bytes = sizeof(int32_t) * 128 * (THREADS / kWarp);
-    static constexpr size_t bytes = vals_bytes + keys_bytes + hist_bytes + sizeof(CtaScratch<THREADS>);
+    static constexpr size_t hi_bytes = WIDE ? (NMAX + 15) / 16 * 16 : 0;
+    static constexpr size_t bytes =
+        vals_bytes + keys_bytes + hist_bytes + hi_bytes + sizeof(CtaScratch<THREADS>);
     static_assert(bytes <= 232448, "an ESC CTA bin's shared memory exceeds 227 KB");
 };
 
 // SKIP_LE > 0: rows of at most SKIP_LE products are left to a smaller kernel
 // of the same bin; SKIP_GT: rows of more than NMAX products are left to a
 // larger one (instead of being reported).
-template<typename V, int THREADS, int NMAX, int SKIP_LE = 0, bool SKIP_GT = false>
+template<typename V, int THREADS, int NMAX, int SKIP_LE = 0, bool SKIP_GT = false,
+         bool WIDE = false>
 __global__ __launch_bounds__(THREADS) void k_esc_cta(ProductArgs p) {
-    using L = EscCtaLayout<V, THREADS, NMAX>;
+    using L = EscCtaLayout<V, THREADS, NMAX, WIDE>;
     constexpr int SHIFT = L::SHIFT;
     constexpr uint32_t QMASK = (1u << SHIFT) - 1u;
     constexpr int NW = THREADS / kWarp;
@@ -514,8 +523,9 @@ __global__ __launch_bounds__(THREADS) void k_esc_cta(ProductArgs p) {
     V* vals = reinterpret_cast<V*>(smem_raw);
     uint32_t* keys = reinterpret_cast<uint32_t*>(smem_raw + L::vals_bytes);
     int32_t* hist = reinterpret_cast<int32_t*>(smem_raw + L::vals_bytes + L::keys_bytes);
+    uint8_t* hi = smem_raw + L::vals_bytes + L::keys_bytes + L::hist_bytes;
     auto& sc = *reinterpret_cast<CtaScratch<THREADS>*>(smem_raw + L::vals_bytes + L::keys_bytes +
-                                                        L::hist_bytes);
+                                                        L::hist_bytes + L::hi_bytes);
     const int tid = threadIdx.x;
     const int row = p.rows[blockIdx.x];
     const int c0 = p.c_rpt[row];
@@ -542,19 +552,25 @@ __global__ __launch_bounds__(THREADS) void k_esc_cta(ProductArgs p) {
                 col = 0;
             }
             keys[q] = (static_cast<uint32_t>(col) << SHIFT) | static_cast<uint32_t>(q);
+            if constexpr (WIDE) hi[q] = static_cast<uint8_t>(static_cast<uint32_t>(col) >> L::LOW);
             vals[q] = kp.prod;
         });
     // the column bits of the keys: B.n - 1 needs this many
     const int colbits = 32 - __clz(p.n_cols > 1 ? p.n_cols - 1 : 1);
-    cta_radix_sort<THREADS, L::RMAX>(keys, nip, SHIFT, colbits, hist, sc.warp_tot);
+    cta_radix_sort<THREADS, L::RMAX>(keys, nip, SHIFT, min(colbits, L::LOW), hist, sc.warp_tot,
+                                     WIDE ? hi : nullptr, QMASK);
+    auto column = [&](uint32_t u) -> uint32_t {
+        if constexpr (WIDE) return (static_cast<uint32_t>(hi[u & QMASK]) << L::LOW) | (u >> SHIFT);
+        else return u >> SHIFT;
+    };
     const int per = (nip + THREADS - 1) / THREADS;
     const int i0 = min(tid * per, nip);
     const int i1 = min(i0 + per, nip);
     int heads = 0;
     {
-        uint32_t prev = i0 > 0 ? (keys[i0 - 1] >> SHIFT) : 0xffffffffu;
+        uint32_t prev = i0 > 0 ? column(keys[i0 - 1]) : 0xffffffffu;
         for (int i = i0; i < i1; i++) {
-            const uint32_t c = keys[i] >> SHIFT;
+            const uint32_t c = column(keys[i]);
             heads += c != prev;
             prev = c;
         }
@@ -564,15 +580,15 @@ __global__ __launch_bounds__(THREADS) void k_esc_cta(ProductArgs p) {
     int r = inc - heads;
     int32_t* out_col = p.c_col + c0;
     V* out_val = static_cast<V*>(p.c_val) + c0;
-    uint32_t prev = i0 > 0 ? (keys[i0 - 1] >> SHIFT) : 0xffffffffu;
+    uint32_t prev = i0 > 0 ? column(keys[i0 - 1]) : 0xffffffffu;
     for (int i = i0; i < i1; i++) {
         const uint32_t u = keys[i];
-        const uint32_t c = u >> SHIFT;
+        const uint32_t c = column(u);
         if (c != prev) {
             V sum = vals[u & QMASK];
             for (int k = i + 1; k < nip; k++) {
                 const uint32_t w = keys[k];
-                if ((w >> SHIFT) != c) break;
+                if (column(w) != c) break;
                 sum += vals[w & QMASK];
             }
             out_col[r] = static_cast<int32_t>(c);
@@ -603,6 +619,7 @@ constexpr int kSampleWarps = 8;
 constexpr int kSampleSlots = 1024;
 constexpr int kSampleProducts = 256;
 constexpr int kSampleMore = 3 * kSampleSlots / 4;
+constexpr int kSampleMoreEntries = 128;
 
 __global__ __launch_bounds__(kSampleWarps * kWarp) void k_esc_sample(ProductArgs p, int32_t m,
                                                                       int32_t samples,
@@ -610,110 +627,152 @@ __global__ __launch_bounds__(kSampleWarps * kWarp) void k_esc_sample(ProductArgs
                                                                       EscSample* out) {
     constexpr unsigned kFull = 0xffffffffu;
     __shared__ int32_t s_tab[kSampleWarps][kSampleSlots];
+    // the CTA's sums, added to `out` with one atomic each (an atomic per row
+    // and sum took 30 us of the sample)
+    __shared__ EscSample s_sum;
     const int lane = threadIdx.x & 31;
     const int wid = threadIdx.x >> 5;
     const int w = blockIdx.x * kSampleWarps + wid;
-    if (w >= samples) return;
-    const int row = static_cast<int>(static_cast<int64_t>(w) * m / samples);
-    const int a0 = p.a_rpt[row];
-    const int a1 = p.a_rpt[row + 1];
-    const int cap = lim.limit[kEscBins - 1];
-    auto add = [&](int64_t* to, int64_t v) {
-        atomicAdd(reinterpret_cast<unsigned long long*>(to), static_cast<unsigned long long>(v));
-    };
-    auto count_nip = [&](int64_t v, bool above) {
-        if (lane == 0) {
-            add(&out->nip_seen, v);
-            if (above) add(&out->nip_above, v);
+    static_assert(sizeof(EscSample) % sizeof(int32_t) == 0, "words");
+    constexpr int kWords = sizeof(EscSample) / sizeof(int32_t);
+    for (int i = threadIdx.x; i < kWords; i += kSampleWarps * kWarp)
+        reinterpret_cast<int32_t*>(&s_sum)[i] = 0;
+    __syncthreads();
+    auto sample = [&](EscSample* sum) {
+        const int row = static_cast<int>(static_cast<int64_t>(w) * m / samples);
+        const int a0 = p.a_rpt[row];
+        const int a1 = p.a_rpt[row + 1];
+        const int cap = lim.limit[kEscBins - 1];
+        auto add = [&](int64_t* to, int64_t v) {
+            atomicAdd(reinterpret_cast<unsigned long long*>(to), static_cast<unsigned long long>(v));
+        };
+        auto count_nip = [&](int64_t v, bool above) {
+            if (lane == 0) {
+                add(&sum->nip_seen, v);
+                if (above) add(&sum->nip_above, v);
+            }
+        };
+        if (a1 - a0 > cap) {  // more products than the team bins take (>= a1 - a0)
+            count_nip(a1 - a0, true);
+            return;
         }
-    };
-    if (a1 - a0 > cap) {  // more products than the team bins take (>= a1 - a0)
-        count_nip(a1 - a0, true);
-        return;
-    }
-    long long nip_ll = 0;
-    int lo = INT32_MAX;
-    int hi = -1;
-    for (int e = a0 + lane; e < a1; e += kWarp) {
-        const int c = __ldg(p.a_col + e);
-        const int s0 = __ldg(p.b_rpt + c);
-        const int s1 = __ldg(p.b_rpt + c + 1);
-        nip_ll += s1 - s0;
-        if (s0 < s1) {
-            lo = min(lo, __ldg(p.b_col + s0));
-            hi = max(hi, __ldg(p.b_col + s1 - 1));
+        long long nip_ll = 0;
+        for (int e = a0 + lane; e < a1; e += kWarp) {
+            const int c = __ldg(p.a_col + e);
+            nip_ll += __ldg(p.b_rpt + c + 1) - __ldg(p.b_rpt + c);
         }
-    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) nip_ll += __shfl_xor_sync(kFull, nip_ll, o);
-    if (nip_ll == 0) return;
-    count_nip(nip_ll, nip_ll > cap);
-    if (nip_ll > kSampleMaxNip) return;
-    const int nip = static_cast<int>(nip_ll);
-    lo = __reduce_min_sync(kFull, lo);
-    hi = __reduce_max_sync(kFull, hi);
-    int b = 0;
-    while (b < kEscBins && nip > lim.limit[b]) b++;
-    int32_t* tab = s_tab[wid];
-    for (int i = lane; i < kSampleSlots; i += kWarp) tab[i] = kEmpty;
-    __syncwarp();
-    int fresh = 0;
-    // the A entries [from, to): their first `most` products past `done`
-    auto insert = [&](int from, int to, int done, int most) {
-        team_for_products_at<kWarp>(p.a_col, p.b_rpt, from, to, [&](int qb, int, int q) {
-            if (done + q < most)
-                fresh += table_insert(tab, kSampleSlots, __ldg(p.b_col + qb), p.status, row);
-        });
-        return __reduce_add_sync(kFull, fresh);
-    };
-    // the entries that hold the first `most` products: [a0, cut), and the
-    // products in them
-    auto cut_at = [&](int most, int& products) {
-        int run = 0;
-        for (int base = a0; base < a1; base += kWarp) {
-            const int e = base + lane;
-            int len = 0;
-            if (e < a1) {
+        for (int o = 16; o > 0; o >>= 1) nip_ll += __shfl_xor_sync(kFull, nip_ll, o);
+        if (nip_ll == 0) return;
+        count_nip(nip_ll, nip_ll > cap);
+        // (a row past the team bins of many entries would set the sample's time)
+        if (nip_ll > kSampleMaxNip || (nip_ll > cap && a1 - a0 > kSampleMoreEntries)) return;
+        const int nip = static_cast<int>(nip_ll);
+        int b = 0;
+        while (b < kEscBins && nip > lim.limit[b]) b++;
+        int32_t* tab = s_tab[wid];
+        for (int i = lane; i < kSampleSlots; i += kWarp) tab[i] = kEmpty;
+        __syncwarp();
+        int fresh = 0;
+        // the A entries [from, to): their first `most` products past `done`
+        auto insert = [&](int from, int to, int done, int most) {
+            team_for_products_at<kWarp>(p.a_col, p.b_rpt, from, to, [&](int qb, int, int q) {
+                if (done + q < most)
+                    fresh += table_insert(tab, kSampleSlots, __ldg(p.b_col + qb), p.status, row);
+            }, most - done);
+            return __reduce_add_sync(kFull, fresh);
+        };
+        // the entries that hold the first `most` products: [a0, cut), and the
+        // products in them
+        auto cut_at = [&](int most, int& products) {
+            int run = 0;
+            for (int base = a0; base < a1; base += kWarp) {
+                const int e = base + lane;
+                int len = 0;
+                if (e < a1) {
+                    const int c = __ldg(p.a_col + e);
+                    len = __ldg(p.b_rpt + c + 1) - __ldg(p.b_rpt + c);
+                }
+                const int inc = team_inclusive_scan<kWarp>(kFull, len, lane);
+                const unsigned hit = __ballot_sync(kFull, run + inc >= most);
+                if (hit != 0u) {
+                    const int at = __ffs(hit) - 1;
+                    products = run + __shfl_sync(kFull, inc, at);
+                    return base + at + 1;
+                }
+                run += __shfl_sync(kFull, inc, kWarp - 1);
+            }
+            products = run;
+            return a1;
+        };
+        int seen = nip;
+        const int cut = nip > kSampleProducts ? cut_at(kSampleProducts, seen) : a1;
+        const int first_nip = min(nip, kSampleProducts);
+        const int first = insert(a0, cut, 0, kSampleProducts);
+        int all_nip = first_nip;
+        int all = first;
+        const bool repeats = 4 * first_nip >= 5 * first;
+        // the row's column span (sorted B rows): of rows that repeat columns and of
+        // short ones, where it costs one load more
+        int lo = INT32_MAX;
+        int hi = -1;
+        if (repeats || a1 - a0 <= kWarp) {
+            for (int e = a0 + lane; e < a1; e += kWarp) {
                 const int c = __ldg(p.a_col + e);
-                len = __ldg(p.b_rpt + c + 1) - __ldg(p.b_rpt + c);
+                const int s0 = __ldg(p.b_rpt + c);
+                const int s1 = __ldg(p.b_rpt + c + 1);
+                if (s0 < s1) {
+                    lo = min(lo, __ldg(p.b_col + s0));
+                    hi = max(hi, __ldg(p.b_col + s1 - 1));
+                }
             }
-            const int inc = team_inclusive_scan<kWarp>(kFull, len, lane);
-            const unsigned hit = __ballot_sync(kFull, run + inc >= most);
-            if (hit != 0u) {
-                const int at = __ffs(hit) - 1;
-                products = run + __shfl_sync(kFull, inc, at);
-                return base + at + 1;
-            }
-            run += __shfl_sync(kFull, inc, kWarp - 1);
+            lo = __reduce_min_sync(kFull, lo);
+            hi = __reduce_max_sync(kFull, hi);
         }
-        products = run;
-        return a1;
+        // repeats in the first products: walk on (whole B rows; the table holds
+        // kSampleMore columns at most)
+        if (nip > kSampleProducts && repeats) {
+            int done = seen;
+            const int cut2 = nip > kSampleMore ? cut_at(kSampleMore, done) : a1;
+            // (the cut row's products past kSampleProducts were skipped above)
+            all = insert(cut, cut2, seen, kSampleMore);
+            all_nip = min(nip, kSampleMore) - (seen - kSampleProducts);
+        }
+        if (lane == 0) {
+            if (b < kEscBins) {
+                add(&sum->nip[b], first_nip);
+                add(&sum->nnz[b], first);
+            }
+            add(&sum->all_nip[b], all_nip);
+            add(&sum->all_nnz[b], all);
+            add(&sum->row_nip[b], nip);
+            add(&sum->rows[b], 1);
+            if (hi >= lo) atomicMax(&sum->span[b], hi - lo + 1);
+        }
     };
-    int seen = nip;
-    const int cut = nip > kSampleProducts ? cut_at(kSampleProducts, seen) : a1;
-    const int first_nip = min(nip, kSampleProducts);
-    const int first = insert(a0, cut, 0, kSampleProducts);
-    int all_nip = first_nip;
-    int all = first;
-    // repeats in the first products: walk on (whole B rows; the table holds
-    // kSampleMore columns at most)
-    if (nip > kSampleProducts && 4 * first_nip >= 5 * first) {
-        int done = seen;
-        const int cut2 = nip > kSampleMore ? cut_at(kSampleMore, done) : a1;
-        // (the cut row's products past kSampleProducts were skipped above)
-        all = insert(cut, cut2, seen, kSampleMore);
-        all_nip = min(nip, kSampleMore) - (seen - kSampleProducts);
+    if (w < samples) sample(&s_sum);
+    __syncthreads();
+    const int t = threadIdx.x;
+    auto flush = [&](const int64_t* from, int64_t* to) {
+        if (*from != 0)
+            atomicAdd(reinterpret_cast<unsigned long long*>(to),
+                      static_cast<unsigned long long>(*from));
+    };
+    if (t < kEscBins) {
+        flush(&s_sum.nip[t], &out->nip[t]);
+        flush(&s_sum.nnz[t], &out->nnz[t]);
     }
-    if (lane == 0) {
-        if (b < kEscBins) {
-            add(&out->nip[b], first_nip);
-            add(&out->nnz[b], first);
-        }
-        add(&out->all_nip[b], all_nip);
-        add(&out->all_nnz[b], all);
-        add(&out->row_nip[b], nip);
-        add(&out->rows[b], 1);
-        if (hi >= lo) atomicMax(&out->span[b], hi - lo + 1);
+    if (t >= 32 && t <= 32 + kEscBins) {
+        const int c = t - 32;
+        flush(&s_sum.all_nip[c], &out->all_nip[c]);
+        flush(&s_sum.all_nnz[c], &out->all_nnz[c]);
+        flush(&s_sum.row_nip[c], &out->row_nip[c]);
+        flush(&s_sum.rows[c], &out->rows[c]);
+        if (s_sum.span[c] > 0) atomicMax(&out->span[c], s_sum.span[c]);
+    }
+    if (t == 64) {
+        flush(&s_sum.nip_seen, &out->nip_seen);
+        flush(&s_sum.nip_above, &out->nip_above);
     }
 }
 
@@ -806,6 +865,9 @@ __global__ __launch_bounds__(THREADS) void k_s2n_cta_spill(ProductArgs p) {
 // the set bits before it in at most 4 words, all independent reads --
 // instead of a binary search; values accumulate with global reductions into
 // C.val.  Then each thread clears its non-empty words and summary word.
+// A wider B is taken in ranges of 2^20 columns, the row's two walks once per
+// range (the one-pass ladder of a wide B; its hash tables of 43,008 slots took
+// longer than two ranges do).
 // (4-word blocks rather than 8: 0.289 -> 0.280 ms on the 1M power-law
 // product, for 16 KB more shared memory.)  The cluster bin below keeps
 // 8-word blocks in the same layout (its rank table uses half the space).
@@ -822,7 +884,8 @@ struct BitmapLayout {
     static_assert(kSummaryWords == THREADS, "one summary word per thread");
 };
 
-template<typename V, int THREADS, int CAP>
+// RANGES: B.n > 2^20 (the range loop costs the one-range kernel 7 %).
+template<typename V, int THREADS, int CAP, bool RANGES>
 __global__ __launch_bounds__(THREADS) void k_s2n_bitmap(ProductArgs p) {
     using L = BitmapLayout<V, THREADS, CAP>;
     constexpr int NW = THREADS / kWarp;
@@ -833,11 +896,7 @@ __global__ __launch_bounds__(THREADS) void k_s2n_bitmap(ProductArgs p) {
     auto& sc = *reinterpret_cast<CtaScratch<THREADS>*>(smem_raw + L::bm_bytes +
                                                         L::summary_bytes + L::rank_bytes);
     const int tid = threadIdx.x;
-    const int words = (p.n_cols + 31) >> 5;
-    if (words > kBitmapWords) {
-        if (tid == 0 && blockIdx.x < p.nrows) report(p.status, kStCapacity, p.rows[blockIdx.x], 0);
-        return;
-    }
+    const int words = min((p.n_cols + 31) >> 5, kBitmapWords);
     __shared__ int32_t s_rid;  // the row this CTA takes next
     for (int i = tid; i < words; i += THREADS) bm[i] = 0u;
     summary[tid] = 0u;
@@ -864,64 +923,71 @@ __global__ __launch_bounds__(THREADS) void k_s2n_bitmap(ProductArgs p) {
             copy_scaled_b_row<V>(p, row, a0, c0, tid, THREADS);
             continue;
         }
-        cta_for_products_mlp<THREADS, kBitmapWalkU>(
-            p.a_col, p.b_rpt, a0, a1, sc, [&](int qb, int, int) { return __ldg(p.b_col + qb); },
-            [&](int32_t key, int, int, int) {
-                if (static_cast<uint32_t>(key) >= static_cast<uint32_t>(p.n_cols)) {
-                    report(p.status, kStBadInput, row, key);  // outside the bitmap
-                    return;
-                }
-                const int wi = key >> 5;
-                if (atomicOr(bm + wi, 1u << (key & 31)) == 0u)
-                    atomicOr(summary + (wi >> 5), 1u << (wi & 31));
-            });
-        const uint32_t sw = summary[tid];
-        int cnt = 0;
-        for (uint32_t m = sw; m != 0u; m &= m - 1u) cnt += __popc(bm[w0 + __ffs(m) - 1]);
-        const int inc = block_inclusive_scan<THREADS>(cnt, sc.warp_tot);
-        const int total = sc.warp_tot[NW - 1];
-        int pos = inc - cnt;
-        int32_t* cols = p.c_col + c0;
+        int done = 0;  // the row's columns before this range
+        for (int c_next = 0; RANGES ? c_next < p.n_cols : c_next == 0; c_next += kBitmapCols) {
+            const int c_lo = RANGES ? c_next : 0;
+            const unsigned range =
+                RANGES ? static_cast<unsigned>(min(kBitmapCols, p.n_cols - c_lo)) : p.n_cols;
+            cta_for_products_mlp<THREADS, kBitmapWalkU>(
+                p.a_col, p.b_rpt, a0, a1, sc, [&](int qb, int, int) { return __ldg(p.b_col + qb); },
+                [&](int32_t col, int, int, int) {
+                    const unsigned key = static_cast<unsigned>(col) - static_cast<unsigned>(c_lo);
+                    if (key >= range) {  // in another range, or outside B
+                        if (!RANGES || static_cast<uint32_t>(col) >= static_cast<uint32_t>(p.n_cols))
+                            report(p.status, kStBadInput, row, col);
+                        return;
+                    }
+                    const int wi = key >> 5;
+                    if (atomicOr(bm + wi, 1u << (key & 31)) == 0u)
+                        atomicOr(summary + (wi >> 5), 1u << (wi & 31));
+                });
+            const uint32_t sw = summary[tid];
+            int cnt = 0;
+            for (uint32_t m = sw; m != 0u; m &= m - 1u) cnt += __popc(bm[w0 + __ffs(m) - 1]);
+            const int inc = block_inclusive_scan<THREADS>(cnt, sc.warp_tot);
+            const int total = sc.warp_tot[NW - 1];
+            int pos = (RANGES ? done : 0) + inc - cnt;
+            int32_t* cols = p.c_col + c0;
 #pragma unroll
-        for (int bb = 0; bb < 8; bb++) {
-            block_rank[(w0 >> 2) + bb] = pos;
-            for (uint32_t m = (sw >> (4 * bb)) & 0xfu; m != 0u; m &= m - 1u) {
-                const int wi = w0 + 4 * bb + __ffs(m) - 1;
-                for (uint32_t word = bm[wi]; word != 0u; word &= word - 1u) {
-                    if (pos < bound) cols[pos] = wi * 32 + __ffs(word) - 1;
-                    pos++;
+            for (int bb = 0; bb < 8; bb++) {
+                block_rank[(w0 >> 2) + bb] = pos;
+                for (uint32_t m = (sw >> (4 * bb)) & 0xfu; m != 0u; m &= m - 1u) {
+                    const int wi = w0 + 4 * bb + __ffs(m) - 1;
+                    for (uint32_t word = bm[wi]; word != 0u; word &= word - 1u) {
+                        if (pos < bound) cols[pos] = c_lo + wi * 32 + __ffs(word) - 1;
+                        pos++;
+                    }
                 }
             }
-        }
-        int nnz = bound;
-        if (p.row_nnz != nullptr) {  // one-pass: the count is the row's nnz
-            nnz = total <= bound ? total : bound;
-            if (tid == 0) p.row_nnz[row] = nnz;
-        } else if (total != nnz && tid == 0) {
-            report(p.status, kStCapacity, row, total);
-        }
-        V* out = static_cast<V*>(p.c_val) + c0;
-        for (int i = tid; i < nnz; i += THREADS) out[i] = V(0);
-        __syncthreads();
-        cta_for_products_mlp<THREADS, kBitmapWalkU>(
-            p.a_col, p.b_rpt, a0, a1, sc,
-            [&](int qb, int ai, int) {
-                return KeyProduct<V>{__ldg(p.b_col + qb), ldv<V>(p.a_val, ai) * ldv<V>(p.b_val, qb)};
-            },
-            [&](const KeyProduct<V>& kp, int, int, int) {
-                const int32_t key = kp.key;
-                if (static_cast<uint32_t>(key) >= static_cast<uint32_t>(p.n_cols)) return;
-                const int wi = key >> 5;
-                const int w4 = wi & ~3;
-                int rank = block_rank[wi >> 2] + __popc(bm[wi] & ((1u << (key & 31)) - 1u));
+            const int nnz = min((RANGES ? done : 0) + total, bound);  // through this range
+            V* out = static_cast<V*>(p.c_val) + c0;
+            for (int i = (RANGES ? done : 0) + tid; i < nnz; i += THREADS) out[i] = V(0);
+            __syncthreads();
+            cta_for_products_mlp<THREADS, kBitmapWalkU>(
+                p.a_col, p.b_rpt, a0, a1, sc,
+                [&](int qb, int ai, int) {
+                    return KeyProduct<V>{__ldg(p.b_col + qb), ldv<V>(p.a_val, ai) * ldv<V>(p.b_val, qb)};
+                },
+                [&](const KeyProduct<V>& kp, int, int, int) {
+                    const unsigned key = static_cast<unsigned>(kp.key) - static_cast<unsigned>(c_lo);
+                    if (key >= range) return;
+                    const int wi = key >> 5;
+                    const int w4 = wi & ~3;
+                    int rank = block_rank[wi >> 2] + __popc(bm[wi] & ((1u << (key & 31)) - 1u));
 #pragma unroll
-                for (int t = 0; t < 3; t++)
-                    if (w4 + t < wi) rank += __popc(bm[w4 + t]);
-                if (rank < nnz) atomicAdd(out + rank, kp.prod);
-            });
-        for (uint32_t m = sw; m != 0u; m &= m - 1u) bm[w0 + __ffs(m) - 1] = 0u;
-        summary[tid] = 0u;
-        __syncthreads();
+                    for (int t = 0; t < 3; t++)
+                        if (w4 + t < wi) rank += __popc(bm[w4 + t]);
+                    if (rank < nnz) atomicAdd(out + rank, kp.prod);
+                });
+            for (uint32_t m = sw; m != 0u; m &= m - 1u) bm[w0 + __ffs(m) - 1] = 0u;
+            summary[tid] = 0u;
+            done += total;
+            __syncthreads();
+        }
+        if (tid == 0) {
+            if (p.row_nnz != nullptr) p.row_nnz[row] = min(done, bound);  // one pass
+            else if (done != bound) report(p.status, kStCapacity, row, done);
+        }
     }
 }
 
@@ -1182,7 +1248,14 @@ cudaError_t launch_esc_warp(const ProductArgs& p, cudaStream_t s) {
 
 template<typename V, int THREADS, int NMAX>
 cudaError_t launch_esc_cta(const ProductArgs& p, cudaStream_t s) {
-    k_esc_cta<V, THREADS, NMAX><<<p.nrows, THREADS, EscCtaLayout<V, THREADS, NMAX>::bytes, s>>>(p);
+    using L = EscCtaLayout<V, THREADS, NMAX, true>;
+    if (static_cast<int64_t>(p.n_cols) > (int64_t(1) << L::LOW))
+        k_esc_cta<V, THREADS, NMAX, 0, false, true><<<p.nrows, THREADS, L::bytes, s>>>(p);
+    else if constexpr (L::LOW >= ilog2(kBitmapCols))
+        k_esc_cta<V, THREADS, NMAX>
+            <<<p.nrows, THREADS, EscCtaLayout<V, THREADS, NMAX>::bytes, s>>>(p);
+    else
+        k_esc_cta<V, THREADS, NMAX, 0, false, true><<<p.nrows, THREADS, L::bytes, s>>>(p);
     return cudaGetLastError();
 }
 
@@ -1191,8 +1264,12 @@ cudaError_t launch_esc_cta(const ProductArgs& p, cudaStream_t s) {
 // (so the slot sizes must not be overwritten by the fill: row_slot is null).
 template<typename V>
 cudaError_t launch_esc_cta_split(const ProductArgs& p, cudaStream_t s) {
-    k_esc_cta<V, 256, 3072, kEscCtaSmall, false>
-        <<<p.nrows, 256, EscCtaLayout<V, 256, 3072>::bytes, s>>>(p);
+    if (p.n_cols > kBitmapCols)
+        k_esc_cta<V, 256, 3072, kEscCtaSmall, false, true>
+            <<<p.nrows, 256, EscCtaLayout<V, 256, 3072, true>::bytes, s>>>(p);
+    else
+        k_esc_cta<V, 256, 3072, kEscCtaSmall, false>
+            <<<p.nrows, 256, EscCtaLayout<V, 256, 3072>::bytes, s>>>(p);
     if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
     k_esc_cta<V, 128, kEscCtaSmall, 0, true>
         <<<p.nrows, 128, EscCtaLayout<V, 128, kEscCtaSmall>::bytes, s>>>(p);
@@ -1284,7 +1361,9 @@ cudaError_t launch_bitmap(const ProductArgs& p, cudaStream_t s) {
             return e;
         }
     }
-    k_s2n_bitmap<V, THREADS, CAP><<<grid, THREADS, BitmapLayout<V, THREADS, CAP>::bytes, s>>>(p);
+    constexpr size_t bytes = BitmapLayout<V, THREADS, CAP>::bytes;
+    if (p.n_cols > kBitmapCols) k_s2n_bitmap<V, THREADS, CAP, true><<<grid, THREADS, bytes, s>>>(p);
+    else k_s2n_bitmap<V, THREADS, CAP, false><<<grid, THREADS, bytes, s>>>(p);
     return cudaGetLastError();
 }
 
@@ -1436,14 +1515,18 @@ const BinLauncher EscSplitBin<V>::entry = {BinKind::Team, kEscSplit, 8, 256,
 
 template<typename V>
 struct EscCtaBins {
-    static const BinLauncher entries[2];
+    static const BinLauncher entries[4];
 };
 template<typename V>
-const BinLauncher EscCtaBins<V>::entries[2] = {
+const BinLauncher EscCtaBins<V>::entries[4] = {
     {BinKind::Cta, kEscCtaSmall, 1, 128, EscCtaLayout<V, 128, kEscCtaSmall>::bytes,
      "esc_cta128_n1024", launch_esc_cta<V, 128, kEscCtaSmall>},
     {BinKind::Cta, 3072, 1, 256, EscCtaLayout<V, 256, 3072>::bytes, "esc_cta256_n3072",
      launch_esc_cta<V, 256, 3072>},
+    {BinKind::Cta, 12288, 1, 1024, EscCtaLayout<V, 1024, 12288, true>::bytes, "esc_cta1024_n12288",
+     launch_esc_cta<V, 1024, 12288>},
+    {BinKind::Cta, kBitmapCols, 1, 1024, BitmapLayout<V, 1024, kBitmapCols>::bytes,
+     "s2n_bitmap1024_ranges", launch_bitmap<V, 1024, kBitmapCols>},
 };
 
 template<typename V>
@@ -1461,12 +1544,22 @@ cudaError_t prepare_one() {
     B200_SMEM((k_s2n_cta_spill<V, 256, 4096, 3072>), (CtaLayout<256, 4096, 3072>::bytes));
     B200_SMEM((k_s2n_cta<V, 512, 16384, 12288>), (CtaLayout<512, 16384, 12288>::bytes));
     B200_SMEM((k_s2n_cta<V, 1024, 43008, 32768>), (CtaLayout<1024, 43008, 32768>::bytes));
-    B200_SMEM((k_s2n_bitmap<V, 1024, kBitmapCols>), (BitmapLayout<V, 1024, kBitmapCols>::bytes));
+    B200_SMEM((k_s2n_bitmap<V, 1024, kBitmapCols, false>),
+              (BitmapLayout<V, 1024, kBitmapCols>::bytes));
+    B200_SMEM((k_s2n_bitmap<V, 1024, kBitmapCols, true>),
+              (BitmapLayout<V, 1024, kBitmapCols>::bytes));
     B200_SMEM((k_s2n_bitmap_cluster<V, 1024>), (BitmapLayout<V, 1024, kBitmapCols>::bytes));
     B200_SMEM((k_esc_team<V, 32, 256, 768>), (EscLayout<V, 32, 256, 768>::bytes));
     B200_SMEM((k_esc_team<V, 32, 256, kEscSplit>), (EscLayout<V, 32, 256, kEscSplit>::bytes));
     B200_SMEM((k_esc_cta<V, 256, 3072>), (EscCtaLayout<V, 256, 3072>::bytes));
     B200_SMEM((k_esc_cta<V, 128, kEscCtaSmall>), (EscCtaLayout<V, 128, kEscCtaSmall>::bytes));
+    B200_SMEM((k_esc_cta<V, 128, kEscCtaSmall, 0, false, true>),
+              (EscCtaLayout<V, 128, kEscCtaSmall, true>::bytes));
+    B200_SMEM((k_esc_cta<V, 256, 3072, 0, false, true>), (EscCtaLayout<V, 256, 3072, true>::bytes));
+    B200_SMEM((k_esc_cta<V, 256, 3072, kEscCtaSmall, false, true>),
+              (EscCtaLayout<V, 256, 3072, true>::bytes));
+    B200_SMEM((k_esc_cta<V, 1024, 12288, 0, false, true>),
+              (EscCtaLayout<V, 1024, 12288, true>::bytes));
     B200_SMEM((k_esc_cta<V, 256, 3072, kEscCtaSmall, false>), (EscCtaLayout<V, 256, 3072>::bytes));
     B200_SMEM((k_esc_cta<V, 128, kEscCtaSmall, 0, true>), (EscCtaLayout<V, 128, kEscCtaSmall>::bytes));
 #undef B200_SMEM

@@ -115,6 +115,9 @@ constexpr int kBitmapCols = 1 << 20;
 constexpr int64_t kClusterBitmapCols = int64_t(8) * kBitmapCols;
 int s2n_bitmap_ladder_f64(const BinLauncher** out);
 int s2n_bitmap_ladder_f32(const BinLauncher** out);
+// Expanding, sorting and compressing packs a column, a product's place and, in
+// the warp bins, a row into one 32-bit key: B.n up to this.
+constexpr int kEscCols = 1 << 22;
 // One-pass ladder for B.n <= kBitmapCols (key = NIP of the row): the warp,
 // team and 256-thread bins expand, sort and compress; then the bitmap ladder's
 // bitmap and global bins.  Same bin count and limits as the bitmap ladder.
@@ -129,6 +132,8 @@ const BinLauncher* s2n_esc_split_bin_f32();
 // (half the fixed cost of each radix pass and scan, twice the CTAs per SM:
 // 1M power-law product, the bin 0.233 -> 0.223 ms serialised).
 constexpr int kEscCtaSmall = 1024;
+// which = 2, 3: a wide B's one-pass rows of up to 12,288 products (1,024
+// threads), and above (the bitmap bin over ranges of columns).
 const BinLauncher* s2n_esc_cta_f64(int which);
 const BinLauncher* s2n_esc_cta_f32(int which);
 

@@ -216,10 +216,14 @@ __device__ __forceinline__ void cta_sort_swz(int32_t* keys, int n) {
 // (digit, warp) gives every key its place.  `hist` holds 128 * THREADS / 32
 // ints.  All threads must call it.  Equal digits keep their order, so keys
 // whose low bits hold their input position come out ordered by the sort bits
-// and then by position.
+// and then by position.  With `hi` given, one more pass follows on the digits
+// hi[key & hi_mask]: bits above the key's 32, kept beside the keys by their
+// low bits.
 template<int THREADS, int RMAX>
 __device__ __forceinline__ void cta_radix_sort(uint32_t* keys, int n, int lo_bit, int nbits,
-                                               int32_t* hist, int32_t* warp_tot) {
+                                               int32_t* hist, int32_t* warp_tot,
+                                               const uint8_t* hi = nullptr,
+                                               uint32_t hi_mask = 0u) {
     constexpr int NW = THREADS / kWarp;
     constexpr int DIGITS = 128;
     static_assert(NW * DIGITS == 4 * THREADS, "four counters per thread in the scan");
@@ -230,7 +234,13 @@ __device__ __forceinline__ void cta_radix_sort(uint32_t* keys, int n, int lo_bit
     const int S = kWarp * ((n + THREADS - 1) / THREADS);
     const int R = S / kWarp;  // <= RMAX
     int32_t* wh = hist + w * DIGITS;
-    for (int bit = lo_bit; bit < lo_bit + nbits; bit += 7) {
+    const int passes = (nbits + 6) / 7;
+    for (int pass = 0; pass < passes + (hi != nullptr ? 1 : 0); pass++) {
+        const int bit = lo_bit + 7 * pass;
+        auto digit = [&](uint32_t key) -> unsigned {
+            if (hi != nullptr && pass == passes) return hi[key & hi_mask];
+            return (key >> bit) & (DIGITS - 1);
+        };
         uint32_t k[RMAX];
         int rk[RMAX];
 #pragma unroll
@@ -245,7 +255,7 @@ __device__ __forceinline__ void cta_radix_sort(uint32_t* keys, int n, int lo_bit
         for (int i = 0; i < RMAX; i++) {
             if (i < R) {
                 const bool valid = w * S + kWarp * i + lane < n;
-                const unsigned d = (k[i] >> bit) & (DIGITS - 1);
+                const unsigned d = digit(k[i]);
                 unsigned peers = __ballot_sync(0xffffffffu, valid);
 #pragma unroll
                 for (int b = 0; b < 7; b++) {
@@ -280,7 +290,7 @@ __device__ __forceinline__ void cta_radix_sort(uint32_t* keys, int n, int lo_bit
 #pragma unroll
         for (int i = 0; i < RMAX; i++) {
             if (i < R && w * S + kWarp * i + lane < n) {
-                const unsigned d = (k[i] >> bit) & (DIGITS - 1);
+                const unsigned d = digit(k[i]);
                 keys[wh[d] + rk[i]] = k[i];
             }
         }

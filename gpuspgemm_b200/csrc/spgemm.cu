@@ -692,7 +692,7 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     // Its sums come back with the fill binning's plan: they choose one pass
     // or two and, per fill bin, expand-sort-compress or hashing.
     const Ladder ladf = make_ladder(fil, nfil, h->min_num_bin);
-    const int esc_mode = (narrow && h->esc != 2) ? h->esc : 2;
+    const int esc_mode = (n <= kEscCols && h->esc != 2) ? h->esc : 2;
     const bool sampled = A->nnz >= kSampleMinNnz &&
                          (h->esc != 2 || (cr == nullptr && h->one_pass == 0));
     if (sampled) {
@@ -930,7 +930,7 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
             return bail(cuda_fail(e_, what));                            \
         }                                                                \
     } while (0)
-        // B.n <= 2^20: fill bins may expand, sort and compress instead of
+        // B.n <= 2^22: fill bins may expand, sort and compress instead of
         // hashing (same limits, so the binning does not depend on it)
         BinLauncher one_fil[16];
         for (int b = 0; b < nfil && b < 16; b++) one_fil[b] = fil[b];
@@ -1003,6 +1003,14 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
                     h->info.esc_mask |= 1 << b;
                 }
             }
+        }
+        // a wide B's larger rows where the team bins' rows repeat few columns:
+        // sorting by a CTA of 1,024, then the bitmap in column ranges, instead
+        // of hash tables
+        if (split && !narrow) {
+            for (int which = 2; which <= 3; which++)
+                one_fil[kEscBins - 1 + which] =
+                    sizeof(V) == 8 ? *s2n_esc_cta_f64(which) : *s2n_esc_cta_f32(which);
         }
         // the fill bins' rows (append binning counts by finer lists)
         int32_t bin_rows[kMaxBins] = {};
