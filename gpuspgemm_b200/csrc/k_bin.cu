@@ -1128,4 +1128,29 @@ cudaError_t launch_total_nip(const int32_t* a_rpt, const int32_t* a_col, const i
     return cudaGetLastError();
 }
 
+namespace {
+
+// Copies `words` words to page-locked host memory and then raises `flag` there
+// to `seq`: the host, which polls the flag, sees the words and knows that the
+// stream's earlier work is done.  One CTA.
+__global__ __launch_bounds__(256) void k_publish(const uint32_t* __restrict__ src, int32_t words,
+                                                 uint32_t* __restrict__ dst,
+                                                 unsigned long long* __restrict__ flag,
+                                                 unsigned long long seq) {
+    for (int i = threadIdx.x; i < words; i += 256) dst[i] = src[i];
+    __threadfence_system();
+    __syncthreads();
+    if (threadIdx.x == 0) *reinterpret_cast<volatile unsigned long long*>(flag) = seq;
+}
+
+}  // namespace
+
+cudaError_t launch_publish(const void* src, size_t bytes, void* dst, unsigned long long* flag,
+                           unsigned long long seq, cudaStream_t s) {
+    k_publish<<<1, 256, 0, s>>>(static_cast<const uint32_t*>(src),
+                                static_cast<int32_t>(bytes / sizeof(uint32_t)),
+                                static_cast<uint32_t*>(dst), flag, seq);
+    return cudaGetLastError();
+}
+
 }  // namespace b200

@@ -297,6 +297,9 @@ cudaError_t launch_compact_rows(const int32_t* off, const int32_t* rpt, int32_t 
 // when the sampled rows' NIP / nnz is at most this; a C with more spare
 // capacity than this factor is then copied to arrays of its size.
 constexpr double kCapSlack = 1.1;
+// `bytes` (a multiple of 4) to page-locked host memory, then *flag = seq there.
+cudaError_t launch_publish(const void* src, size_t bytes, void* dst, unsigned long long* flag,
+                           unsigned long long seq, cudaStream_t s);
 // Operand validation (checked mode).
 cudaError_t launch_check_csr(const int32_t* rpt, const int32_t* col, int32_t m, int32_t n,
                              int32_t nnz, DevStatus* st, cudaStream_t s);

@@ -14,6 +14,7 @@
 // creates/destroys its streams and scratch in every call (setup.cuh:164-165,
 // cleanup.cuh:15-31); here streams, events and scratch live in the handle.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -124,6 +125,8 @@ struct spgemm_handle_s {
     size_t slots_bytes = 0;
     b200::HostMirror* mirror = nullptr;  // pinned
     char* front_host = nullptr;          // pinned copy of the scratch front
+    unsigned long long* flag = nullptr;  // pinned: the last publish seen (front_host's last word)
+    unsigned long long published = 0;    // the last publish queued
     // host-operand staging on the device
     void* in_buf = nullptr;
     size_t in_bytes = 0;
@@ -357,15 +360,42 @@ spgemm_status mirror_finish(spgemm_handle_s* h, const Plan* plan, const Scratch&
     return SPGEMM_OK;
 }
 
+// One synchronisation: a one-CTA kernel behind the stream's work writes the
+// scratch front to page-locked memory and raises a flag the host polls.  From
+// the last kernel's end to the host's next launch that takes ~8 us where a
+// copy and cudaStreamSynchronize took ~19, which a small product pays three
+// times.  (With profiling on the stream is synchronised: its events are read.)
+spgemm_status publish_and_wait(spgemm_handle_s* h, cudaStream_t stream, const Scratch& s) {
+    const char* dev0 = static_cast<const char*>(h->scratch);
+    const size_t front = static_cast<size_t>(reinterpret_cast<const char*>(s.scan_state) - dev0);
+    if (front > kFrontBytes - sizeof(*h->flag))
+        return fail(SPGEMM_ERR_INTERNAL, "scratch front exceeds its mirror");
+    const unsigned long long seq = ++h->published;
+    B200_TRY(launch_publish(h->scratch, front, h->front_host, h->flag, seq, stream));
+    h->info.host_syncs++;
+    if (h->profile) {
+        B200_TRY(cudaStreamSynchronize(stream));
+        return SPGEMM_OK;
+    }
+    const volatile unsigned long long* flag = h->flag;
+    for (unsigned spins = 1; *flag != seq; spins++) {
+        if ((spins & 0xfffu) != 0u) continue;
+        // every few tens of microseconds: has the stream failed?
+        const cudaError_t e = cudaStreamQuery(stream);
+        if (e == cudaErrorNotReady) continue;
+        if (e != cudaSuccess) return cuda_fail(e, "wait for the stream");
+        if (*flag == seq) break;
+        return fail(SPGEMM_ERR_INTERNAL, "the stream ended without publishing its state");
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    return SPGEMM_OK;
+}
+
 spgemm_status sync_mirror(spgemm_handle_s* h, cudaStream_t stream, const Plan* plan,
                           const Scratch& s, bool with_sample = false,
                           const Plan* plan_b = nullptr) {
     const char* dev0 = static_cast<const char*>(h->scratch);
-    const size_t front = static_cast<size_t>(reinterpret_cast<const char*>(s.scan_state) - dev0);
-    if (front > kFrontBytes) return fail(SPGEMM_ERR_INTERNAL, "scratch front exceeds its mirror");
-    B200_TRY(cudaMemcpyAsync(h->front_host, h->scratch, front, cudaMemcpyDeviceToHost, stream));
-    B200_TRY(cudaStreamSynchronize(stream));
-    h->info.host_syncs++;
+    if (spgemm_status st = publish_and_wait(h, stream, s); st != SPGEMM_OK) return st;
     auto at = [&](const void* dev) {
         return h->front_host + (static_cast<const char*>(dev) - dev0);
     };
@@ -1205,10 +1235,8 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
             }));
         }
         release();
-        if (cudaError_t e = cudaStreamSynchronize(stream); e != cudaSuccess)
-            return bail(cuda_fail(e, "final synchronize"));
+        B200_ONE(publish_and_wait(h, stream, s));
         mark(6);
-        h->info.host_syncs++;
         resolve_profile(h);
         return SPGEMM_OK;
         }
@@ -1467,14 +1495,18 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
             }));
     }
     mark(5);
-    if (cudaError_t e = cudaMemcpyAsync(&h->mirror->status, fill_status, sizeof(DevStatus),
-                                        cudaMemcpyDeviceToHost, stream);
-        e != cudaSuccess)
-        return bail(cuda_fail(e, "read status"));
-    if (cudaError_t e = cudaStreamSynchronize(stream); e != cudaSuccess)
-        return bail(cuda_fail(e, "final synchronize"));
+    if (fill_status == s.status) {
+        B200_STEP(sync_mirror(h, stream, scan_plan, s));
+    } else {
+        if (cudaError_t e = cudaMemcpyAsync(&h->mirror->status, fill_status, sizeof(DevStatus),
+                                            cudaMemcpyDeviceToHost, stream);
+            e != cudaSuccess)
+            return bail(cuda_fail(e, "read status"));
+        if (cudaError_t e = cudaStreamSynchronize(stream); e != cudaSuccess)
+            return bail(cuda_fail(e, "final synchronize"));
+        h->info.host_syncs++;
+    }
     mark(6);
-    h->info.host_syncs++;
     B200_STEP(status_to_error(h->mirror->status));
     resolve_profile(h);
 #undef B200_STEP
@@ -1967,11 +1999,7 @@ spgemm_status transpose(spgemm_handle_s* h, const spgemm_csr_view* A, spgemm_csr
     B200_STEP(launch_bins(h, tl, ntl, 4, plan, s.bins2, pa, stream));
     B200_CUDA(cudaFreeAsync(keys, stream), "free transpose records");
     keys = nullptr;
-    B200_CUDA(cudaMemcpyAsync(&h->mirror->status, s.status, sizeof(DevStatus),
-                              cudaMemcpyDeviceToHost, stream),
-              "read status");
-    B200_CUDA(cudaStreamSynchronize(stream), "final synchronize");
-    h->info.host_syncs++;
+    B200_STEP(sync_mirror(h, stream, s.plan2, s));
     B200_STEP(status_to_error(h->mirror->status));
     resolve_profile(h);
 #undef B200_CUDA
@@ -2349,6 +2377,8 @@ spgemm_status spgemm_create(spgemm_handle_t* handle, int device) {
     B200_TRY(cudaEventCreateWithFlags(&h->ev_front, cudaEventDisableTiming));
     B200_TRY(cudaMallocHost(reinterpret_cast<void**>(&h->mirror), sizeof(HostMirror)));
     B200_TRY(cudaMallocHost(reinterpret_cast<void**>(&h->front_host), kFrontBytes));
+    h->flag = reinterpret_cast<unsigned long long*>(h->front_host + kFrontBytes) - 1;
+    *h->flag = 0;
     if (spgemm_status st = device_pool(dev, &h->pool); st != SPGEMM_OK) return st;
     *handle = h;
     return SPGEMM_OK;
