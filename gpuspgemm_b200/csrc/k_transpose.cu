@@ -8,17 +8,19 @@
 //      which nothing else needs yet);
 //   2. the product path's binning pass with the scan (k_bin.cu) turns the
 //      counts into T.rpt and bins T's rows by length;
-//   3. scatter: entry (i, j) of A at position e goes to place T.rpt[j] + rank
-//      as one 16-byte record: the key (i << 32 | e) and the value;
-//   4. each row's records are put in key order (the keys are unique, so the
-//      order is fully determined) and written as T.col = i, T.val: rows of up
-//      to kTrFlat entries by counting, per record, the row's smaller keys;
+//   3. scatter: entry (i, j) of A at position e puts e at place T.rpt[j] + rank
+//      and i at row_of[e];
+//   4. each row's positions are put in ascending order -- A's entries are in
+//      row order, so that is the order of the rows i, and of equal ones by
+//      position -- and T.col = row_of[e], T.val = A.val[e] written: rows of up to
+//      kTrFlat entries by counting, per entry, the row's smaller positions;
 //      longer rows by sorting.
-// Bound by random 32-byte sectors: one atomic and one record write per entry,
-// whatever the record's size up to 32 bytes, so the value travels with the key
-// instead of being gathered after the sort.  Entries are dealt to lanes flat
-// (a warp per row of A left most lanes idle at 5.5 entries a row, and took a
-// second atomic per entry).
+// Bound by random 32-byte sectors: per entry an atomic, a 4-byte write and two
+// 4- or 8-byte gathers.  The write is 4 bytes so that its array stays in L2 until
+// its sectors are whole: with 16-byte records (key and value, no gathers) the
+// scatter of 5.5 M entries took 0.152 ms and 85 MB of DRAM reads to fill partly
+// written sectors.  Entries are dealt to lanes flat (a warp per row of A left
+// most lanes idle at 5.5 entries a row, and took a second atomic per entry).
 // Sorting uses the bitonic network in which every comparator sends the
 // smaller key to the lower index; a row of len keys runs the network of the
 // next power of two with the missing tail taken as +infinity, and every
@@ -30,29 +32,18 @@ namespace b200 {
 
 namespace {
 
-// One entry on its way to its row of T: key = row of A << 32 | position in A,
-// val = the bits of the value.
-struct __align__(16) TrRec {
-    uint64_t key;
-    uint64_t val;
-};
-
-__device__ __forceinline__ uint64_t sort_key(uint64_t x) { return x; }
-__device__ __forceinline__ uint64_t sort_key(const TrRec& x) { return x.key; }
-
-template<typename T>
-__device__ __forceinline__ void cas_asc(T* a, long long lo, long long hi) {
-    const T x = a[lo];
-    const T y = a[hi];
-    if (sort_key(x) > sort_key(y)) {
+__device__ __forceinline__ void cas_asc(uint32_t* a, long long lo, long long hi) {
+    const uint32_t x = a[lo];
+    const uint32_t y = a[hi];
+    if (x > y) {
         a[lo] = y;
         a[hi] = x;
     }
 }
 
 // Ascending sort of a[0, len) by the CTA (a in shared or global memory).
-template<int THREADS, typename T>
-__device__ void cta_sort_keys(T* a, long long len) {
+template<int THREADS>
+__device__ void cta_sort_keys(uint32_t* a, long long len) {
     long long N = 1;
     while (N < len) N <<= 1;
     const long long pairs = N >> 1;
@@ -76,20 +67,11 @@ __device__ void cta_sort_keys(T* a, long long len) {
     }
 }
 
-__host__ __device__ __forceinline__ const TrRec* recs_of(const ProductArgs& p) {
-    return reinterpret_cast<const TrRec*>(p.keys);
-}
-
+// One entry of T at `at`: A's entry e.
 template<typename V>
-__device__ __forceinline__ uint64_t val_bits(V v) {
-    if constexpr (sizeof(V) == 8) return static_cast<uint64_t>(__double_as_longlong(v));
-    else return __float_as_uint(v);
-}
-
-template<typename V>
-__device__ __forceinline__ V val_of(uint64_t bits) {
-    if constexpr (sizeof(V) == 8) return __longlong_as_double(static_cast<long long>(bits));
-    else return __uint_as_float(static_cast<uint32_t>(bits));
+__device__ __forceinline__ void store_entry(const ProductArgs& p, int32_t at, uint32_t e) {
+    p.c_col[at] = __ldg(p.tr_row + e);
+    static_cast<V*>(p.c_val)[at] = __ldg(static_cast<const V*>(p.a_val) + e);
 }
 
 // ---- 1. column counts and ranks ---------------------------------------------
@@ -97,6 +79,8 @@ __device__ __forceinline__ V val_of(uint64_t bits) {
 // atomics (any order: step 4 sorts).  A column index outside [0, n) is not
 // counted and its rank is -1; the host sees the total fall short of nnz and
 // reports the operand as invalid.  kCountUnroll atomics per lane in flight.
+// Bound by L2 atomics that return a value: 5.5 M in 0.051 ms, with lanes of one
+// column grouped by __match_any_sync (as here, for hot columns) or not.
 constexpr int kCountUnroll = 4;
 
 __global__ __launch_bounds__(256) void k_col_count(const int32_t* __restrict__ col, int32_t nnz,
@@ -135,7 +119,7 @@ __global__ __launch_bounds__(256) void k_col_count(const int32_t* __restrict__ c
     }
 }
 
-// ---- 3. scatter of records --------------------------------------------------
+// ---- 3. scatter of positions --------------------------------------------------
 // A warp takes kScatterTile consecutive entries of A, finds the rows of the
 // first and the last by a 32-way search of A.rpt, and each lane finds its
 // entries' rows by a binary search between them.  Entries whose column is
@@ -161,14 +145,13 @@ __device__ __forceinline__ int warp_row_of(const int32_t* __restrict__ rpt, int3
     return lo;
 }
 
-template<typename V>
 __global__ __launch_bounds__(256) void k_tr_scatter(const int32_t* __restrict__ a_rpt,
-                                                    const int32_t* __restrict__ a_col,
-                                                    const V* __restrict__ a_val, int32_t m,
+                                                    const int32_t* __restrict__ a_col, int32_t m,
                                                     int32_t nnz,
                                                     const int32_t* __restrict__ t_rpt,
                                                     const int32_t* __restrict__ rank,
-                                                    TrRec* __restrict__ recs) {
+                                                    uint32_t* __restrict__ perm,
+                                                    int32_t* __restrict__ row_of) {
     const int lane = threadIdx.x & 31;
     const long long tile = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) +
                            (threadIdx.x >> 5);
@@ -191,50 +174,46 @@ __global__ __launch_bounds__(256) void k_tr_scatter(const int32_t* __restrict__ 
     for (int k = 0; k < kScatterPer; k++) {
         const int e = static_cast<int>(e0 + k * kWarp + lane);
         if (pos[k] < 0) continue;
+        perm[pos[k]] = static_cast<uint32_t>(e);
         int lo = rlo;
         for (int len = rhi - rlo + 1; len > 1;) {
             const int half = len >> 1;
             lo = __ldg(a_rpt + lo + half) <= e ? lo + half : lo;
             len -= half;
         }
-        recs[pos[k]] = TrRec{(static_cast<uint64_t>(static_cast<uint32_t>(lo)) << 32) |
-                                 static_cast<uint32_t>(e),
-                             val_bits<V>(__ldg(a_val + e))};
+        row_of[e] = lo;
     }
 }
 
-// ---- 4. the rows' records in key order ---------------------------------------
-// Rows of up to kTrFlat records: a warp takes rows_per_warp consecutive rows of
-// T and walks their records flat, a lane per record; the record's place in its
-// row is the number of smaller keys there (one broadcast read per record of
+// ---- 4. the rows' entries in order ---------------------------------------------
+// Rows of up to kTrFlat entries: a warp takes rows_per_warp consecutive rows of
+// T and walks their entries flat, a lane per entry; the entry's place in its
+// row is the number of smaller positions there (one broadcast read per entry of
 // the row, most from L1: cheaper than a warp's sorting network for the short
-// rows of a graph and free of its 64-bit shuffles).  It runs over all rows and
-// leaves the longer ones to their bins' kernels.
+// rows of a graph).  It runs over all rows and leaves the longer ones to their
+// bins' kernels.
 constexpr int kTrFlat = 128;
 
 template<typename V>
-__global__ __launch_bounds__(256) void k_tr_place(const int32_t* __restrict__ t_rpt, int32_t n,
-                                                  int32_t rows_per_warp,
-                                                  const TrRec* __restrict__ recs,
-                                                  int32_t* __restrict__ t_col,
-                                                  V* __restrict__ t_val) {
+__global__ __launch_bounds__(256) void k_tr_place(ProductArgs p, int32_t rows_per_warp) {
     constexpr unsigned kFull = 0xffffffffu;
     const int lane = threadIdx.x & 31;
+    const uint32_t* __restrict__ perm = reinterpret_cast<const uint32_t*>(p.keys);
     const long long r0 = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) +
                           (threadIdx.x >> 5)) * rows_per_warp;
-    if (r0 >= n) return;  // uniform over the warp
+    if (r0 >= p.n_cols) return;  // uniform over the warp
     int t0 = 0;
     int len = 0;
-    if (lane < rows_per_warp && r0 + lane < n) {
-        t0 = __ldg(t_rpt + r0 + lane);
-        len = __ldg(t_rpt + r0 + lane + 1) - t0;
+    if (lane < rows_per_warp && r0 + lane < p.n_cols) {
+        t0 = __ldg(p.c_rpt + r0 + lane);
+        len = __ldg(p.c_rpt + r0 + lane + 1) - t0;
         if (len > kTrFlat) len = 0;
     }
     const int inc = team_inclusive_scan<kWarp>(kFull, len, lane);
     const int total = __shfl_sync(kFull, inc, 31);
     for (int f0 = 0; f0 < total; f0 += kWarp) {  // uniform over the warp
         const int f = f0 + lane;
-        // record f's row: the first lane with inc > f
+        // entry f's row: the first lane with inc > f
         int j = -1;
 #pragma unroll
         for (int step = 16; step >= 1; step >>= 1) {
@@ -246,28 +225,23 @@ __global__ __launch_bounds__(256) void k_tr_place(const int32_t* __restrict__ t_
         const int before = __shfl_sync(kFull, inc - len, j);
         const int count = __shfl_sync(kFull, len, j);
         if (f < total) {
-            const TrRec mine = recs[start + (f - before)];
+            const uint32_t mine = __ldg(perm + start + (f - before));
+            const int32_t row = __ldg(p.tr_row + mine);
+            const V val = __ldg(static_cast<const V*>(p.a_val) + mine);
             int place = 0;
 #pragma unroll 4
-            for (int i = 0; i < count; i++) place += __ldg(&recs[start + i].key) < mine.key;
-            t_col[start + place] = static_cast<int32_t>(mine.key >> 32);
-            t_val[start + place] = val_of<V>(mine.val);
+            for (int i = 0; i < count; i++) place += __ldg(perm + start + i) < mine;
+            p.c_col[start + place] = row;
+            static_cast<V*>(p.c_val)[start + place] = val;
         }
     }
-}
-
-template<typename V>
-__device__ __forceinline__ void store_entry(const ProductArgs& p, int32_t at, uint64_t key) {
-    p.c_col[at] = static_cast<int32_t>(key >> 32);
-    static_cast<V*>(p.c_val)[at] =
-        __ldg(static_cast<const V*>(p.a_val) + static_cast<uint32_t>(key & 0xffffffffu));
 }
 
 // Rows of up to CAP keys: one CTA per row, the keys in shared memory.
 template<typename V, int THREADS, int CAP>
 __global__ __launch_bounds__(THREADS) void k_tr_sort_cta(ProductArgs p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    uint64_t* s = reinterpret_cast<uint64_t*>(smem_raw);
+    uint32_t* s = reinterpret_cast<uint32_t*>(smem_raw);
     const int row = p.rows[blockIdx.x];
     const int t0 = p.c_rpt[row];
     const int len = p.c_rpt[row + 1] - t0;
@@ -275,13 +249,13 @@ __global__ __launch_bounds__(THREADS) void k_tr_sort_cta(ProductArgs p) {
         if (threadIdx.x == 0) report(p.status, kStCapacity, row, len);
         return;
     }
-    for (int i = threadIdx.x; i < len; i += THREADS) s[i] = recs_of(p)[t0 + i].key;
+    for (int i = threadIdx.x; i < len; i += THREADS) s[i] = reinterpret_cast<const uint32_t*>(p.keys)[t0 + i];
     __syncthreads();
     cta_sort_keys<THREADS>(s, len);
     for (int i = threadIdx.x; i < len; i += THREADS) store_entry<V>(p, t0 + i, s[i]);
 }
 
-// Longer rows: one CTA per row, sorting the row's records in place in global
+// Longer rows: one CTA per row, sorting the row's positions in place in global
 // memory (the network's passes stay in L2 for rows of a few MB).
 template<typename V, int THREADS>
 __global__ __launch_bounds__(THREADS) void k_tr_sort_global(ProductArgs p) {
@@ -289,17 +263,14 @@ __global__ __launch_bounds__(THREADS) void k_tr_sort_global(ProductArgs p) {
         const int row = p.rows[rid];
         const int t0 = p.c_rpt[row];
         const int len = p.c_rpt[row + 1] - t0;
-        TrRec* a = reinterpret_cast<TrRec*>(p.keys) + t0;
+        uint32_t* a = reinterpret_cast<uint32_t*>(p.keys) + t0;
         cta_sort_keys<THREADS>(a, len);
-        for (int i = threadIdx.x; i < len; i += THREADS) {
-            p.c_col[t0 + i] = static_cast<int32_t>(a[i].key >> 32);
-            static_cast<V*>(p.c_val)[t0 + i] = val_of<V>(a[i].val);
-        }
+        for (int i = threadIdx.x; i < len; i += THREADS) store_entry<V>(p, t0 + i, a[i]);
         __syncthreads();
     }
 }
 
-// Rows per warp of k_tr_place for about kPlaceEntries records a warp.
+// Rows per warp of k_tr_place for about kPlaceEntries entries a warp.
 constexpr int64_t kPlaceEntries = 256;
 
 // Every row of T, not only this bin's list: the list would cost a gather per
@@ -311,14 +282,13 @@ cudaError_t launch_place(const ProductArgs& p, cudaStream_t s) {
     int rows = 1;
     while (rows < kWarp && (2 * rows) * nnz <= kPlaceEntries * n) rows *= 2;
     const int64_t warps = (static_cast<int64_t>(n) + rows - 1) / rows;
-    k_tr_place<V><<<static_cast<unsigned>((warps + 7) / 8), 256, 0, s>>>(
-        p.c_rpt, n, rows, recs_of(p), p.c_col, static_cast<V*>(p.c_val));
+    k_tr_place<V><<<static_cast<unsigned>((warps + 7) / 8), 256, 0, s>>>(p, rows);
     return cudaGetLastError();
 }
 
 template<typename V, int THREADS, int CAP>
 cudaError_t launch_cta(const ProductArgs& p, cudaStream_t s) {
-    k_tr_sort_cta<V, THREADS, CAP><<<p.nrows, THREADS, sizeof(uint64_t) * CAP, s>>>(p);
+    k_tr_sort_cta<V, THREADS, CAP><<<p.nrows, THREADS, sizeof(uint32_t) * CAP, s>>>(p);
     return cudaGetLastError();
 }
 
@@ -337,9 +307,9 @@ struct TransposeLadder {
 template<typename V>
 const BinLauncher TransposeLadder<V>::bins[4] = {
     {BinKind::Team, kTrFlat, 8, 256, 0, "tr_place", launch_place<V>},
-    {BinKind::Cta, 2048, 1, 256, sizeof(uint64_t) * 2048, "tr_sort_cta2048",
+    {BinKind::Cta, 2048, 1, 256, sizeof(uint32_t) * 2048, "tr_sort_cta2048",
      launch_cta<V, 256, 2048>},
-    {BinKind::Cta, 16384, 1, 1024, sizeof(uint64_t) * 16384, "tr_sort_cta16384",
+    {BinKind::Cta, 16384, 1, 1024, sizeof(uint32_t) * 16384, "tr_sort_cta16384",
      launch_cta<V, 1024, 16384>},
     {BinKind::Global, INT32_MAX, 1, 1024, 0, "tr_sort_global", launch_global<V, 1024>},
 };
@@ -348,7 +318,7 @@ template<typename V>
 cudaError_t prepare_ladder() {
     cudaError_t e = cudaFuncSetAttribute(k_tr_sort_cta<V, 1024, 16384>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(sizeof(uint64_t) * 16384));
+                                         static_cast<int>(sizeof(uint32_t) * 16384));
     return e;
 }
 
@@ -379,19 +349,13 @@ cudaError_t launch_col_count(const int32_t* col, int32_t nnz, int32_t n, int32_t
     return cudaGetLastError();
 }
 
-cudaError_t launch_tr_scatter(const int32_t* a_rpt, const int32_t* a_col, const void* a_val,
-                              int value_bytes, int32_t m, int32_t nnz, const int32_t* t_rpt,
-                              const int32_t* rank, uint64_t* recs, cudaStream_t s) {
+cudaError_t launch_tr_scatter(const int32_t* a_rpt, const int32_t* a_col, int32_t m, int32_t nnz,
+                              const int32_t* t_rpt, const int32_t* rank, uint32_t* perm,
+                              int32_t* row_of, cudaStream_t s) {
     if (m <= 0 || nnz <= 0) return cudaSuccess;
     constexpr int kPerCta = 8 * kScatterTile;
     const unsigned g = static_cast<unsigned>((static_cast<long long>(nnz) + kPerCta - 1) / kPerCta);
-    TrRec* out = reinterpret_cast<TrRec*>(recs);
-    if (value_bytes == 8)
-        k_tr_scatter<double><<<g, 256, 0, s>>>(a_rpt, a_col, static_cast<const double*>(a_val), m,
-                                               nnz, t_rpt, rank, out);
-    else
-        k_tr_scatter<float><<<g, 256, 0, s>>>(a_rpt, a_col, static_cast<const float*>(a_val), m,
-                                              nnz, t_rpt, rank, out);
+    k_tr_scatter<<<g, 256, 0, s>>>(a_rpt, a_col, m, nnz, t_rpt, rank, perm, row_of);
     return cudaGetLastError();
 }
 

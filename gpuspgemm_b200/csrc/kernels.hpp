@@ -55,9 +55,10 @@ struct ProductArgs {
     int32_t cluster;        // CTAs per cluster
     int32_t* fail_rows;     // rows that spilled out of a cluster table
     int32_t* fail_count;
-    // transpose: a 16-byte record per entry of T, its first word (row of A << 32
-    // | position in A); n_cols and words are then T's rows and entries
-    uint64_t* keys;
+    // transpose: a 32-bit position in A per entry of T, and the row of A of each
+    // entry of A; n_cols and words are then T's rows and entries
+    uint32_t* keys;
+    const int32_t* tr_row;
     // one-pass fill: c_rpt gives each row a slot of its NIP entries (an upper
     // bound); the kernel writes the row's exact nnz here (nullptr: c_rpt is
     // C's exact row pointer)
@@ -318,11 +319,10 @@ int transpose_ladder_f32(const BinLauncher** out);
 cudaError_t transpose_prepare();
 cudaError_t launch_col_count(const int32_t* col, int32_t nnz, int32_t n, int32_t* cnt,
                              int32_t* rank, cudaStream_t s);
-// recs: kTrRecBytes per entry of A
-constexpr size_t kTrRecBytes = 16;
-cudaError_t launch_tr_scatter(const int32_t* a_rpt, const int32_t* a_col, const void* a_val,
-                              int value_bytes, int32_t m, int32_t nnz, const int32_t* t_rpt,
-                              const int32_t* rank, uint64_t* recs, cudaStream_t s);
+// perm: the entries' positions by T's rows; row_of: the entries' rows of A
+cudaError_t launch_tr_scatter(const int32_t* a_rpt, const int32_t* a_col, int32_t m, int32_t nnz,
+                              const int32_t* t_rpt, const int32_t* rank, uint32_t* perm,
+                              int32_t* row_of, cudaStream_t s);
 // NIP of many independent pairs in one launch (spgemm_get_nip_many).
 struct NipPair {
     const int32_t* a_col;   // A_i's column indices (nnz entries)

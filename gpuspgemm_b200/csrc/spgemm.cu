@@ -1901,7 +1901,7 @@ spgemm_status transpose(spgemm_handle_s* h, const spgemm_csr_view* A, spgemm_csr
     h->info.n_num_bins = ntl;
     B200_TRY(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&T->rpt),
                                      sizeof(int32_t) * (size_t(n) + 1), h->pool, stream));
-    uint64_t* keys = nullptr;
+    uint32_t* keys = nullptr;  // per entry: its position, then its row of A
     auto bail = [&](spgemm_status st) {
         const std::string msg = g_last_error;
         cudaStreamSynchronize(stream);
@@ -1969,11 +1969,11 @@ spgemm_status transpose(spgemm_handle_s* h, const spgemm_csr_view* A, spgemm_csr
         }));
     }
     B200_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&keys),
-                                      kTrRecBytes * size_t(nnz), h->pool, stream),
-              "allocate transpose records");
+                                      2 * sizeof(uint32_t) * size_t(nnz), h->pool, stream),
+              "allocate transpose positions");
+    int32_t* row_of = reinterpret_cast<int32_t*>(keys + nnz);
     B200_STEP(timed(h, "tr_scatter", 3, -1, m, stream, [&](cudaStream_t ss) {
-        return launch_tr_scatter(A->rpt, A->col, A->val, static_cast<int>(sizeof(V)), m, nnz,
-                                 T->rpt, T->col, keys, ss);
+        return launch_tr_scatter(A->rpt, A->col, m, nnz, T->rpt, T->col, keys, row_of, ss);
     }));
     B200_CUDA(cudaMallocFromPoolAsync(&T->val, sizeof(V) * size_t(nnz), h->pool, stream),
               "allocate T.val");
@@ -1994,10 +1994,11 @@ spgemm_status transpose(spgemm_handle_s* h, const spgemm_csr_view* A, spgemm_csr
     pa.c_val = T->val;
     pa.status = s.status;
     pa.keys = keys;
+    pa.tr_row = row_of;
     pa.n_cols = n;
     pa.words = nnz;
     B200_STEP(launch_bins(h, tl, ntl, 4, plan, s.bins2, pa, stream));
-    B200_CUDA(cudaFreeAsync(keys, stream), "free transpose records");
+    B200_CUDA(cudaFreeAsync(keys, stream), "free transpose positions");
     keys = nullptr;
     B200_STEP(sync_mirror(h, stream, s.plan2, s));
     B200_STEP(status_to_error(h->mirror->status));
