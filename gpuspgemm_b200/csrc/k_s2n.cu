@@ -1515,10 +1515,10 @@ const BinLauncher EscSplitBin<V>::entry = {BinKind::Team, kEscSplit, 8, 256,
 
 template<typename V>
 struct EscCtaBins {
-    static const BinLauncher entries[4];
+    static const BinLauncher entries[5];
 };
 template<typename V>
-const BinLauncher EscCtaBins<V>::entries[4] = {
+const BinLauncher EscCtaBins<V>::entries[5] = {
     {BinKind::Cta, kEscCtaSmall, 1, 128, EscCtaLayout<V, 128, kEscCtaSmall>::bytes,
      "esc_cta128_n1024", launch_esc_cta<V, 128, kEscCtaSmall>},
     {BinKind::Cta, 3072, 1, 256, EscCtaLayout<V, 256, 3072>::bytes, "esc_cta256_n3072",
@@ -1527,6 +1527,8 @@ const BinLauncher EscCtaBins<V>::entries[4] = {
      launch_esc_cta<V, 1024, 12288>},
     {BinKind::Cta, kBitmapCols, 1, 1024, BitmapLayout<V, 1024, kBitmapCols>::bytes,
      "s2n_bitmap1024_ranges", launch_bitmap<V, 1024, kBitmapCols>},
+    {BinKind::Cta, kEscCtaMid, 1, 256, EscCtaLayout<V, 256, kEscCtaMid>::bytes, "esc_cta256_n2048",
+     launch_esc_cta<V, 256, kEscCtaMid>},
 };
 
 template<typename V>
@@ -1553,6 +1555,9 @@ cudaError_t prepare_one() {
     B200_SMEM((k_esc_team<V, 32, 256, kEscSplit>), (EscLayout<V, 32, 256, kEscSplit>::bytes));
     B200_SMEM((k_esc_cta<V, 256, 3072>), (EscCtaLayout<V, 256, 3072>::bytes));
     B200_SMEM((k_esc_cta<V, 128, kEscCtaSmall>), (EscCtaLayout<V, 128, kEscCtaSmall>::bytes));
+    B200_SMEM((k_esc_cta<V, 256, kEscCtaMid>), (EscCtaLayout<V, 256, kEscCtaMid>::bytes));
+    B200_SMEM((k_esc_cta<V, 256, kEscCtaMid, 0, false, true>),
+              (EscCtaLayout<V, 256, kEscCtaMid, true>::bytes));
     B200_SMEM((k_esc_cta<V, 128, kEscCtaSmall, 0, false, true>),
               (EscCtaLayout<V, 128, kEscCtaSmall, true>::bytes));
     B200_SMEM((k_esc_cta<V, 256, 3072, 0, false, true>), (EscCtaLayout<V, 256, 3072, true>::bytes));

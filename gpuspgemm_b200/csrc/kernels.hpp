@@ -128,11 +128,14 @@ int s2n_esc_ladder_f32(const BinLauncher** out);
 // (rows of at most kEscSplit products: a smaller kernel, more CTAs per SM).
 const BinLauncher* s2n_esc_split_bin_f64();
 const BinLauncher* s2n_esc_split_bin_f32();
-// The 256-thread bin's two kernels where its rows come in two lists: rows of
-// at most kEscCtaSmall products on 128 threads (which = 0), the others on 256
-// (half the fixed cost of each radix pass and scan, twice the CTAs per SM:
-// 1M power-law product, the bin 0.233 -> 0.223 ms serialised).
+// The 256-thread bin's kernels where its rows come in lists by size: rows of
+// at most kEscCtaSmall products on 128 threads (which = 0; half the fixed cost
+// of each radix pass and scan, twice the CTAs per SM: 1M power-law product, the
+// bin 0.233 -> 0.223 ms serialised), of at most kEscCtaMid on 256 with eight
+// keys a thread (which = 4; fewer registers: 20-product batch 1.22 -> 1.16 ms,
+// 1M power-law 0.992 -> 0.986), the others on 256 with twelve (which = 1).
 constexpr int kEscCtaSmall = 1024;
+constexpr int kEscCtaMid = 2048;
 // which = 2, 3: a wide B's one-pass rows of up to 12,288 products (1,024
 // threads), and above (the bitmap bin over ranges of columns).
 const BinLauncher* s2n_esc_cta_f64(int which);
@@ -246,7 +249,7 @@ cudaError_t launch_bin_offsets_map(const int32_t* src_hist, int32_t* hist, int32
 // plan zeroed by the caller receives the keys' total and max).  Used up to
 // kAppendMaxRows rows: the lists take kListBins words a row.
 constexpr int32_t kAppendMaxRows = int32_t(1) << 22;
-constexpr int kListBins = 11;
+constexpr int kListBins = 12;
 // key = NIP, written to c_rpt; off (or nullptr) receives each row's slot start
 cudaError_t launch_nip_append(const int32_t* a_rpt, const int32_t* a_col, const int32_t* b_rpt,
                               int32_t m, int32_t* c_rpt, int32_t* off, int32_t* lists,

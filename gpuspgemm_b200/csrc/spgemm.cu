@@ -519,9 +519,10 @@ void list_offsets(Plan* plan, int nb, int32_t m) {
 }
 
 // The limits append binning counts one-pass rows by: the fill ladder's, and,
-// where the fill may expand, sort and compress, kEscSplit and kEscCtaSmall
-// too.  Which kernel takes which list is decided when the sample is known:
-// src[e] is the fill bin limit e comes from (kFromSplit, kFromSmall: inserted).
+// where the fill may expand, sort and compress, kEscSplit, kEscCtaSmall and
+// kEscCtaMid too.  Which kernel takes which list is decided when the sample is
+// known: src[e] is the fill bin limit e comes from (kFromSplit, kFromSmall:
+// inserted).
 constexpr int kFromSplit = -1;
 constexpr int kFromSmall = -2;
 struct ListLadder {
@@ -545,6 +546,7 @@ ListLadder list_ladder(const Ladder& fill, bool esc) {
         };
         if (esc && b == kEscBins - 1) put(kEscSplit, kFromSplit);
         if (esc && b == kEscBins) put(kEscCtaSmall, kFromSmall);
+        if (esc && b == kEscBins) put(kEscCtaMid, kFromSmall);
         put(fill.limit[b], b);
         // rows forced to bin min_bin or above: to the lists past the bin below
         if (b == fill.min_bin - 1) l.lad.min_bin = nb;
@@ -1079,7 +1081,8 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
                 list_ids[e] = b;
                 list_fil[e] = one_fil[b];
                 if (b == kEscBins && split) {
-                    const int which = lists.lad.limit[e] <= kEscCtaSmall ? 0 : 1;
+                    const int32_t limit = lists.lad.limit[e];
+                    const int which = limit <= kEscCtaSmall ? 0 : limit <= kEscCtaMid ? 4 : 1;
                     list_fil[e] = sizeof(V) == 8 ? *s2n_esc_cta_f64(which) : *s2n_esc_cta_f32(which);
                 }
                 h->info.num_bin_rows[b] += pf.bin_size[e];

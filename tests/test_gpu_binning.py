@@ -13,7 +13,7 @@ from gpuspgemm_b200.csr import HostCSR
 
 pytestmark = pytest.mark.gpu
 
-LENGTHS = [0, 1, 12, 13, 48, 49, 192, 193, 512, 513, 768, 769, 1024, 1025, 3072, 3073]
+LENGTHS = [0, 1, 12, 13, 48, 49, 192, 193, 512, 513, 768, 769, 1024, 1025, 2048, 2049, 3072, 3073]
 
 
 @pytest.mark.parametrize("passes", [1, 2])

@@ -10,7 +10,7 @@ from gpuspgemm_b200.csr import HostCSR
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [1, 11, 12, 13, 47, 49, 190, 193, 511, 513, 767, 769, 1023, 1025, 3071, 3073, 12287, 12289,
+SIZES = [1, 11, 12, 13, 47, 49, 190, 193, 511, 513, 767, 769, 1023, 1025, 2047, 2049, 3071, 3073, 12287, 12289,
          30000]
 
 
