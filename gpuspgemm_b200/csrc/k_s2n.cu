@@ -884,10 +884,17 @@ struct BitmapLayout {
     static_assert(kSummaryWords == THREADS, "one summary word per thread");
 };
 
-// RANGES: B.n > 2^20 (the range loop costs the one-range kernel 7 %).
-template<typename V, int THREADS, int CAP, bool RANGES>
+// The kernel for B.n up to 2^20 (32 bitmap words a thread), for a narrower B
+// whose words spread thinner over the threads, and for ranges of a wider B.
+// (One kernel for all took 0.280-0.297 ms where the first takes 0.265: the loops
+// over a thread's words must have their trip count at compile time.)
+enum class BitmapMode { kFull, kSpread, kRanges };
+
+template<typename V, int THREADS, int CAP, BitmapMode MODE>
 __global__ __launch_bounds__(THREADS) void k_s2n_bitmap(ProductArgs p) {
     using L = BitmapLayout<V, THREADS, CAP>;
+    constexpr bool RANGES = MODE == BitmapMode::kRanges;
+    constexpr bool SPREAD = MODE == BitmapMode::kSpread;
     constexpr int NW = THREADS / kWarp;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint32_t* bm = reinterpret_cast<uint32_t*>(smem_raw);
@@ -900,7 +907,14 @@ __global__ __launch_bounds__(THREADS) void k_s2n_bitmap(ProductArgs p) {
     __shared__ int32_t s_rid;  // the row this CTA takes next
     for (int i = tid; i < words; i += THREADS) bm[i] = 0u;
     summary[tid] = 0u;
-    const int w0 = tid * 32;  // this thread's bitmap words [w0, w0 + 32)
+    const int w0 = tid * 32;  // kFull, kRanges: this thread's words [w0, w0 + 32)
+    // kSpread: this thread's 4-word blocks [tid * per, (tid + 1) * per), fewer
+    // than eight, so that a narrower B's columns still spread over the CTA (with
+    // 32 words a thread, the 15,800 columns of a row of 30,000 came from 30
+    // threads: 46 such rows 0.112 -> 0.076 ms)
+    const int per = SPREAD ? max(1, ((words + 3) / 4 + THREADS - 1) / THREADS) : 0;
+    // the non-empty words of block g, a bit each
+    auto filled = [&](int g) { return (summary[g >> 3] >> (4 * (g & 7))) & 0xfu; };
     for (int k = 0;; k++) {
         // rows are taken from the launch's counter as CTAs free up (the list
         // is ordered largest first), so the CTAs finish together
@@ -943,23 +957,40 @@ __global__ __launch_bounds__(THREADS) void k_s2n_bitmap(ProductArgs p) {
                 });
             const uint32_t sw = summary[tid];
             int cnt = 0;
-            for (uint32_t m = sw; m != 0u; m &= m - 1u) cnt += __popc(bm[w0 + __ffs(m) - 1]);
+            if constexpr (SPREAD) {
+                for (int g = tid * per; g < (tid + 1) * per; g++)
+                    for (uint32_t m = filled(g); m != 0u; m &= m - 1u)
+                        cnt += __popc(bm[4 * g + __ffs(m) - 1]);
+            } else {
+                for (uint32_t m = sw; m != 0u; m &= m - 1u) cnt += __popc(bm[w0 + __ffs(m) - 1]);
+            }
             const int inc = block_inclusive_scan<THREADS>(cnt, sc.warp_tot);
             const int total = sc.warp_tot[NW - 1];
             int pos = (RANGES ? done : 0) + inc - cnt;
             int32_t* cols = p.c_col + c0;
-#pragma unroll
-            for (int bb = 0; bb < 8; bb++) {
-                block_rank[(w0 >> 2) + bb] = pos;
-                for (uint32_t m = (sw >> (4 * bb)) & 0xfu; m != 0u; m &= m - 1u) {
-                    const int wi = w0 + 4 * bb + __ffs(m) - 1;
+            auto extract = [&](int g, uint32_t m) {
+                block_rank[g] = pos;
+                for (; m != 0u; m &= m - 1u) {
+                    const int wi = 4 * g + __ffs(m) - 1;
                     for (uint32_t word = bm[wi]; word != 0u; word &= word - 1u) {
                         if (pos < bound) cols[pos] = c_lo + wi * 32 + __ffs(word) - 1;
                         pos++;
                     }
                 }
+            };
+            if constexpr (SPREAD) {
+                for (int g = tid * per; g < (tid + 1) * per; g++) extract(g, filled(g));
+            } else {
+#pragma unroll
+                for (int bb = 0; bb < 8; bb++) extract((w0 >> 2) + bb, (sw >> (4 * bb)) & 0xfu);
             }
             const int nnz = min((RANGES ? done : 0) + total, bound);  // through this range
+            if constexpr (!RANGES) {
+                if (tid == 0) {
+                    if (p.row_nnz != nullptr) p.row_nnz[row] = nnz;  // one pass
+                    else if (total != bound) report(p.status, kStCapacity, row, total);
+                }
+            }
             V* out = static_cast<V*>(p.c_val) + c0;
             for (int i = (RANGES ? done : 0) + tid; i < nnz; i += THREADS) out[i] = V(0);
             __syncthreads();
@@ -979,14 +1010,23 @@ __global__ __launch_bounds__(THREADS) void k_s2n_bitmap(ProductArgs p) {
                         if (w4 + t < wi) rank += __popc(bm[w4 + t]);
                     if (rank < nnz) atomicAdd(out + rank, kp.prod);
                 });
-            for (uint32_t m = sw; m != 0u; m &= m - 1u) bm[w0 + __ffs(m) - 1] = 0u;
+            if constexpr (SPREAD) {
+                for (int g = tid * per; g < (tid + 1) * per; g++)
+                    for (uint32_t m = filled(g); m != 0u; m &= m - 1u)
+                        bm[4 * g + __ffs(m) - 1] = 0u;
+                __syncthreads();  // threads share summary words
+            } else {
+                for (uint32_t m = sw; m != 0u; m &= m - 1u) bm[w0 + __ffs(m) - 1] = 0u;
+            }
             summary[tid] = 0u;
             done += total;
             __syncthreads();
         }
-        if (tid == 0) {
-            if (p.row_nnz != nullptr) p.row_nnz[row] = min(done, bound);  // one pass
-            else if (done != bound) report(p.status, kStCapacity, row, done);
+        if constexpr (RANGES) {
+            if (tid == 0) {
+                if (p.row_nnz != nullptr) p.row_nnz[row] = min(done, bound);  // one pass
+                else if (done != bound) report(p.status, kStCapacity, row, done);
+            }
         }
     }
 }
@@ -1362,8 +1402,12 @@ cudaError_t launch_bitmap(const ProductArgs& p, cudaStream_t s) {
         }
     }
     constexpr size_t bytes = BitmapLayout<V, THREADS, CAP>::bytes;
-    if (p.n_cols > kBitmapCols) k_s2n_bitmap<V, THREADS, CAP, true><<<grid, THREADS, bytes, s>>>(p);
-    else k_s2n_bitmap<V, THREADS, CAP, false><<<grid, THREADS, bytes, s>>>(p);
+    if (p.n_cols > kBitmapCols)
+        k_s2n_bitmap<V, THREADS, CAP, BitmapMode::kRanges><<<grid, THREADS, bytes, s>>>(p);
+    else if (p.n_cols > kBitmapCols / 2)
+        k_s2n_bitmap<V, THREADS, CAP, BitmapMode::kFull><<<grid, THREADS, bytes, s>>>(p);
+    else
+        k_s2n_bitmap<V, THREADS, CAP, BitmapMode::kSpread><<<grid, THREADS, bytes, s>>>(p);
     return cudaGetLastError();
 }
 
@@ -1546,9 +1590,11 @@ cudaError_t prepare_one() {
     B200_SMEM((k_s2n_cta_spill<V, 256, 4096, 3072>), (CtaLayout<256, 4096, 3072>::bytes));
     B200_SMEM((k_s2n_cta<V, 512, 16384, 12288>), (CtaLayout<512, 16384, 12288>::bytes));
     B200_SMEM((k_s2n_cta<V, 1024, 43008, 32768>), (CtaLayout<1024, 43008, 32768>::bytes));
-    B200_SMEM((k_s2n_bitmap<V, 1024, kBitmapCols, false>),
+    B200_SMEM((k_s2n_bitmap<V, 1024, kBitmapCols, BitmapMode::kFull>),
               (BitmapLayout<V, 1024, kBitmapCols>::bytes));
-    B200_SMEM((k_s2n_bitmap<V, 1024, kBitmapCols, true>),
+    B200_SMEM((k_s2n_bitmap<V, 1024, kBitmapCols, BitmapMode::kSpread>),
+              (BitmapLayout<V, 1024, kBitmapCols>::bytes));
+    B200_SMEM((k_s2n_bitmap<V, 1024, kBitmapCols, BitmapMode::kRanges>),
               (BitmapLayout<V, 1024, kBitmapCols>::bytes));
     B200_SMEM((k_s2n_bitmap_cluster<V, 1024>), (BitmapLayout<V, 1024, kBitmapCols>::bytes));
     B200_SMEM((k_esc_team<V, 32, 256, 768>), (EscLayout<V, 32, 256, 768>::bytes));
