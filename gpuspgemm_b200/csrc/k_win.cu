@@ -23,8 +23,8 @@
 // G follows the mean length of the B rows read (a step takes one B row).
 // Measured (B200): a 27-point stencil on 60^3 squared, FP32, 149 M products:
 // hash bin 1.49 ms -> window fill 0.82 ms (71 % issue-active, 3,100 warp
-// instructions a row); R * (A * P) on 100^3: count 0.19 -> 0.08 ms, fill about
-// even (0.31).  A team per row with a hash table and row-by-row sums in it (no
+// instructions a row); R * (A * P) on 100^3: count 0.19 -> 0.08 ms, fill 0.31 ->
+// 0.26.  A team per row with a hash table and row-by-row sums in it (no
 // window) took 1.05 ms on the stencil: 6.5 probe rounds a step.
 #include "cta.cuh"
 #include "fill.cuh"
@@ -235,8 +235,11 @@ __global__ __launch_bounds__(256) void k_win_count(ProductArgs p) {
     else if (lane == 0) p.c_rpt[row] = cnt;
 }
 
+// Four CTAs an SM: FP64 took 79 registers without the bound, three CTAs (R * AP
+// of a 100^3 stencil 0.308 -> 0.264 ms); five spill FP32 (60^3 squared 0.82 ->
+// 0.93 ms).
 template<typename V, int G>
-__global__ __launch_bounds__(256) void k_win_fill(ProductArgs p) {
+__global__ __launch_bounds__(256, 4) void k_win_fill(ProductArgs p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int team = threadIdx.x / G;
     const int lane = team_lane<G>();
