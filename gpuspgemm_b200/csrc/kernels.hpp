@@ -164,7 +164,7 @@ cudaError_t launch_win_spill_f32(const ProductArgs& p, cudaStream_t s);
 // per team bin (rows binned by NIP with `lim`; rows above the last limit are
 // only counted in nip_above).  `p` needs A, B and the status word.
 constexpr int kEscBins = 4;
-constexpr int kEscSamples = 4096;
+constexpr int kEscSamples = 2048;  // (4,096 took the SMs from the NIP pass beside it)
 // A team bin expands, sorts and compresses when its sampled NIP / nnz is at
 // most this (ESC sorts NIP keys where the hash bin sorts nnz; measured
 // crossovers: none up to NIP/nnz 4 for rows of <= 48 products, ~1.45 at

@@ -665,7 +665,7 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     C->rpt = c_rpt;
     auto bail = [&](spgemm_status st) {
         const std::string msg = g_last_error;
-        cudaStreamSynchronize(h->side[0]);  // a compression sample may still read A and B
+        cudaStreamSynchronize(h->side[1]);  // a compression sample may still read A and B
         cudaStreamSynchronize(stream);
         spgemm_csr_free(C, stream);
         cudaStreamSynchronize(stream);
@@ -718,20 +718,26 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     // one launch per binning pass, a row list per bin (k_bin.cu)
     const bool append = m <= kAppendMaxRows;
     const Ladder lad1 = make_ladder(sym, nsym, h->min_sym_bin);
-    // Compression sample (products that may run one pass): it reads A and B
-    // only, so it runs on a side stream beside the NIP pass (forked before
-    // it), then decides the one-pass fill binning's limits on the device.
-    // Its sums come back with the fill binning's plan: they choose one pass
-    // or two and, per fill bin, expand-sort-compress or hashing.
+    // Compression sample: it reads A and B only, so it runs on a side stream
+    // beside the NIP pass (forked before it), but queued behind it and at low
+    // priority: ahead of it, its CTAs took a third of the SMs' threads and the
+    // NIP pass ran in two waves (1M rows: both done at 0.115 ms, now at 0.079;
+    // the product 0.977 -> 0.926 ms).  Past kAppendMaxRows rows it also decides
+    // the one-pass fill binning's limits on the device.  Its sums come back
+    // with the first synchronisation: they choose one pass or two and, per
+    // fill bin, the kernel.
     const Ladder ladf = make_ladder(fil, nfil, h->min_num_bin);
     const int esc_mode = (n <= kEscCols && h->esc != 2) ? h->esc : 2;
     const bool sampled = A->nnz >= kSampleMinNnz &&
                          (h->esc != 2 || (cr == nullptr && h->one_pass == 0));
-    if (sampled) {
+    if (sampled)
+        if (cudaError_t e = cudaEventRecord(h->ev_fork, stream); e != cudaSuccess)
+            return bail(cuda_fail(e, "fork the sample stream"));
+    auto queue_sample = [&]() -> spgemm_status {
         EscLimits el{};
         for (int b = 0; b < kEscBins; b++) el.limit[b] = fil[b].limit;
         const int32_t samples = std::min<int32_t>(m, kEscSamples);
-        cudaStream_t side = h->side[0];
+        cudaStream_t side = h->side[1];
         ProductArgs ps = {};
         ps.a_rpt = A->rpt;
         ps.a_col = A->col;
@@ -739,20 +745,17 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
         ps.b_col = B->col;
         ps.status = s.status;
         // (the sample's sums were zeroed with the scratch front above)
-        if (cudaError_t e = cudaEventRecord(h->ev_fork, stream); e != cudaSuccess)
-            return bail(cuda_fail(e, "fork the sample stream"));
-        if (cudaError_t e = cudaStreamWaitEvent(side, h->ev_fork, 0); e != cudaSuccess)
-            return bail(cuda_fail(e, "fork the sample stream"));
-        B200_STEP(timed(h, "esc_sample", 0, -1, samples, side, [&](cudaStream_t ss) {
+        B200_TRY(cudaStreamWaitEvent(side, h->ev_fork, 0));
+        B200_STEP_R(timed(h, "esc_sample", 0, -1, samples, side, [&](cudaStream_t ss) {
             return launch_esc_sample(ps, m, samples, el, s.sample, ss);
         }));
         if (!append)  // (append binning needs no decision on the device)
-            B200_STEP(timed(h, "esc_decide", 0, -1, 1, side, [&](cudaStream_t ss) {
+            B200_STEP_R(timed(h, "esc_decide", 0, -1, 1, side, [&](cudaStream_t ss) {
                 return launch_esc_decide(s.sample, ladf, esc_mode, s.dladder, ss);
             }));
-        if (cudaError_t e = cudaEventRecord(h->ev_sample, side); e != cudaSuccess)
-            return bail(cuda_fail(e, "join the sample stream"));
-    }
+        B200_TRY(cudaEventRecord(h->ev_sample, side));
+        return SPGEMM_OK;
+    };
     // A product likely to run one pass is binned for the fill right away and
     // decided at the one synchronisation that follows; the count binning then
     // runs only if it turns out two-pass.  Its fill binning scans a copy of
@@ -809,6 +812,7 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
         return launch_nip_hist(A->rpt, A->col, B->rpt, m, c_rpt, off, s.hist1, s.plan1, s.status,
                                lad1, ss, s.hist3, s.cta_sum, nip_counts_fill ? &ladx : nullptr);
     }));
+    if (sampled) B200_STEP(queue_sample());
     auto fill_binning = [&]() -> spgemm_status {
         if (append) {
             if (sampled) B200_TRY(cudaStreamWaitEvent(stream, h->ev_sample, 0));
