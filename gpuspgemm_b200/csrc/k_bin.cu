@@ -194,14 +194,14 @@ __device__ __forceinline__ void append_rows(AppendShared& sh, int bin, int32_t r
     if (bin >= 0) lists[bin * stride + at + __popc(peers & ((1u << lane) - 1u))] = row;
 }
 
-// Per-row keys of the CTA's rows -- warp w's group j holds rows
-// (w * PER + j) * 32 + lane of the CTA -- into the lists, the plan's total and
-// max, and, when `off` is given, each row's slot start: the CTA's slots follow
-// one another from a base taken with one atomic on the total (so slots are in
-// row order only within a CTA's rows; a row's slot holds its key's entries).
-template<int PER>
-__device__ __forceinline__ void append_keys(const int32_t (&key)[PER], long long tot, int32_t row0,
-                                            int32_t m, int32_t* __restrict__ off,
+// The keys of the CTA's kBinThreads rows from row0 on, a row per thread, into
+// the lists, the plan's total and max, and, when `off` is given, each row's slot
+// start: the CTA's slots follow one another from a base taken with one atomic
+// on the total (so slots are in row order only within a CTA's rows; a row's
+// slot holds its key's entries).  (1,024 rows a CTA, for a quarter of the
+// reservations: the NIP pass of 1M rows 0.079 ms, with 256 0.066.)
+__device__ __forceinline__ void append_keys(int32_t key, long long tot, int32_t row0, int32_t m,
+                                            int32_t* __restrict__ off,
                                             int32_t* __restrict__ lists, int64_t stride,
                                             Plan* __restrict__ plan, const Ladder& lad) {
     constexpr int NW = kBinThreads / kWarp;
@@ -211,15 +211,11 @@ __device__ __forceinline__ void append_keys(const int32_t (&key)[PER], long long
     __shared__ long long s_base;
     const int lane = threadIdx.x & 31;
     const int w = threadIdx.x >> 5;
-    int32_t mx = 0;
+    const int bin = key > 0 ? find_bin(lad, key) : -1;
     append_clear(sh);
     __syncthreads();
-#pragma unroll
-    for (int j = 0; j < PER; j++) {
-        mx = max(mx, key[j]);
-        append_count(sh, key[j] > 0 ? find_bin(lad, key[j]) : -1);
-    }
-    mx = __reduce_max_sync(0xffffffffu, mx);
+    append_count(sh, bin);
+    const int32_t mx = __reduce_max_sync(0xffffffffu, key);
     tot = warp_sum_ll(tot);
     if (lane == 0) {
         s_sum[w] = tot;
@@ -245,16 +241,11 @@ __device__ __forceinline__ void append_keys(const int32_t (&key)[PER], long long
     __syncthreads();
     // int arithmetic: it wraps only when the total leaves int32, and then the
     // slots are not used (two passes)
-    int run = static_cast<int>(s_base + s_sum[w]);
-#pragma unroll
-    for (int j = 0; j < PER; j++) {
-        const int32_t r = row0 + (w * PER + j) * kWarp + lane;
-        append_rows(sh, key[j] > 0 ? find_bin(lad, key[j]) : -1, r, lists, stride);
-        if (off != nullptr) {
-            const int inc = team_inclusive_scan<kWarp>(0xffffffffu, key[j], lane);
-            if (r < m) off[r] = run + inc - key[j];
-            run += __shfl_sync(0xffffffffu, inc, kWarp - 1);
-        }
+    const int32_t r = row0 + threadIdx.x;
+    append_rows(sh, bin, r, lists, stride);
+    if (off != nullptr) {
+        const int inc = team_inclusive_scan<kWarp>(0xffffffffu, key, lane);
+        if (r < m) off[r] = static_cast<int>(s_base + s_sum[w]) + inc - key;
     }
 }
 
@@ -263,7 +254,7 @@ __device__ __forceinline__ void append_keys(const int32_t (&key)[PER], long long
 // four rows at a time; longer ones the warp, one after another.  (Bound by the
 // latency of a_col -> b_rpt gathers: the medium class keeps four rows' gathers
 // in flight where the warp-per-row walk had one -- 35,937 rows of 84 entries
-// 0.170 -> 0.02 ms, with 256 rows a CTA instead of 1,024.)
+// 0.170 -> 0.03 ms, with 256 rows a CTA instead of 1,024.)
 constexpr int kNipMedium = 128;
 
 __device__ __forceinline__ long long nip_of_rows(const int32_t* __restrict__ a_col,
@@ -339,70 +330,40 @@ __device__ __forceinline__ long long nip_of_rows(const int32_t* __restrict__ a_c
     return nip;
 }
 
-// Rows per CTA: kBinRowsPerCta from kAppendWide rows on, where that fills the
-// chip (148 SMs x 4 CTAs) and shares the reservations; 256 below.
-constexpr int kAppendPer = kBinRowsPerCta / kBinThreads;
-constexpr int32_t kAppendWide = 148 * 4 * kBinRowsPerCta;
-
-template<int PER>
 __global__ __launch_bounds__(kBinThreads) void k_nip_append(
     const int32_t* __restrict__ a_rpt, const int32_t* __restrict__ a_col,
     const int32_t* __restrict__ b_rpt, int32_t m, int32_t* __restrict__ c_rpt,
     int32_t* __restrict__ off, int32_t* __restrict__ lists, int64_t stride,
     Plan* __restrict__ plan, DevStatus* __restrict__ st, const __grid_constant__ Ladder lad) {
-    const int lane = threadIdx.x & 31;
-    const int w = threadIdx.x >> 5;
-    const int32_t row0 = blockIdx.x * (PER * kBinThreads);
-    int32_t key[PER];
-    long long tot = 0;
-#pragma unroll 1
-    for (int j = 0; j < PER; j++) {
-        const int32_t r = row0 + (w * PER + j) * kWarp + lane;
-        int s0 = 0;
-        int s1 = 0;
-        if (r < m) {
-            s0 = a_rpt[r];
-            s1 = a_rpt[r + 1];
-        }
-        const long long nip = nip_of_rows(a_col, b_rpt, s0, s1);
-        int32_t k = 0;
-        if (r < m) {
-            if (nip > INT32_MAX) {
-                report(st, kStNipOverflow, r);
-                k = INT32_MAX;
-            } else {
-                k = static_cast<int32_t>(nip);
-            }
-            c_rpt[r] = k;
-            tot += nip;
-        }
-#pragma unroll
-        for (int q = 0; q < PER; q++)
-            if (q == j) key[q] = k;
+    const int32_t row0 = blockIdx.x * kBinThreads;
+    const int32_t r = row0 + threadIdx.x;
+    int s0 = 0;
+    int s1 = 0;
+    if (r < m) {
+        s0 = a_rpt[r];
+        s1 = a_rpt[r + 1];
     }
-    append_keys<PER>(key, tot, row0, m, off, lists, stride, plan, lad);
+    const long long nip = nip_of_rows(a_col, b_rpt, s0, s1);
+    int32_t key = static_cast<int32_t>(nip);
+    if (nip > INT32_MAX) {
+        report(st, kStNipOverflow, r);
+        key = INT32_MAX;
+    }
+    if (r < m) c_rpt[r] = key;
+    append_keys(key, nip, row0, m, off, lists, stride, plan, lad);
 }
 
 // The same from keys in memory (a NIP per row that an earlier pass wrote).
-template<int PER>
 __global__ __launch_bounds__(kBinThreads) void k_key_append(const int32_t* __restrict__ keys,
                                                             int32_t m, int32_t* __restrict__ off,
                                                             int32_t* __restrict__ lists,
                                                             int64_t stride,
                                                             Plan* __restrict__ plan,
                                                             const __grid_constant__ Ladder lad) {
-    const int lane = threadIdx.x & 31;
-    const int w = threadIdx.x >> 5;
-    const int32_t row0 = blockIdx.x * (PER * kBinThreads);
-    int32_t key[PER];
-    long long tot = 0;
-#pragma unroll
-    for (int j = 0; j < PER; j++) {
-        const int32_t r = row0 + (w * PER + j) * kWarp + lane;
-        key[j] = r < m ? keys[r] : 0;
-        tot += key[j];
-    }
-    append_keys<PER>(key, tot, row0, m, off, lists, stride, plan, lad);
+    const int32_t row0 = blockIdx.x * kBinThreads;
+    const int32_t r = row0 + threadIdx.x;
+    const int32_t key = r < m ? keys[r] : 0;
+    append_keys(key, key, row0, m, off, lists, stride, plan, lad);
 }
 
 // ---- pass 1': nnz histogram + per-CTA nnz sums ----------------------------
@@ -1039,24 +1000,16 @@ cudaError_t launch_nip_append(const int32_t* a_rpt, const int32_t* a_col, const 
                               int64_t stride, Plan* plan, DevStatus* st, const Ladder& lad,
                               cudaStream_t s) {
     if (m <= 0) return cudaSuccess;
-    if (m >= kAppendWide)
-        k_nip_append<kAppendPer><<<(m - 1) / kBinRowsPerCta + 1, kBinThreads, 0, s>>>(
-            a_rpt, a_col, b_rpt, m, c_rpt, off, lists, stride, plan, st, lad);
-    else
-        k_nip_append<1><<<(m - 1) / kBinThreads + 1, kBinThreads, 0, s>>>(
-            a_rpt, a_col, b_rpt, m, c_rpt, off, lists, stride, plan, st, lad);
+    k_nip_append<<<(m - 1) / kBinThreads + 1, kBinThreads, 0, s>>>(
+        a_rpt, a_col, b_rpt, m, c_rpt, off, lists, stride, plan, st, lad);
     return cudaGetLastError();
 }
 
 cudaError_t launch_key_append(const int32_t* keys, int32_t m, int32_t* off, int32_t* lists,
                               int64_t stride, Plan* plan, const Ladder& lad, cudaStream_t s) {
     if (m <= 0) return cudaSuccess;
-    if (m >= kAppendWide)
-        k_key_append<kAppendPer><<<(m - 1) / kBinRowsPerCta + 1, kBinThreads, 0, s>>>(
-            keys, m, off, lists, stride, plan, lad);
-    else
-        k_key_append<1><<<(m - 1) / kBinThreads + 1, kBinThreads, 0, s>>>(keys, m, off, lists,
-                                                                          stride, plan, lad);
+    k_key_append<<<(m - 1) / kBinThreads + 1, kBinThreads, 0, s>>>(keys, m, off, lists, stride,
+                                                                   plan, lad);
     return cudaGetLastError();
 }
 

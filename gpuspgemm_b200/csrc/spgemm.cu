@@ -240,6 +240,15 @@ spgemm_status ensure_scratch(spgemm_handle_s* h, int32_t m, Scratch* s, cudaStre
     return SPGEMM_OK;
 }
 
+// Clears the scratch front and, behind it, the row-pointer scan's state as far
+// as m rows use it.
+cudaError_t clear_front(spgemm_handle_s* h, const Scratch& s, int32_t m, cudaStream_t stream) {
+    const size_t tiles = std::min<size_t>((size_t(m) + kScanAppendTile - 1) / kScanAppendTile,
+                                          size_t(kScanMaxTiles));
+    const char* end = reinterpret_cast<const char*>(s.scan_state + 1 + tiles);
+    return cudaMemsetAsync(h->scratch, 0, end - static_cast<const char*>(h->scratch), stream);
+}
+
 spgemm_status ensure_bitmaps(spgemm_handle_s* h, int64_t words, int32_t rows, int32_t* nmaps,
                             cudaStream_t stream) {
     const int64_t per_map = words * 4;
@@ -687,10 +696,7 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     Scratch s;
     B200_STEP(ensure_scratch(h, m, &s, stream));
     // status, plans and fail counter are contiguous at the front of the scratch
-    if (cudaError_t e = cudaMemsetAsync(
-            h->scratch, 0, reinterpret_cast<char*>(s.hist1) - static_cast<char*>(h->scratch),
-            stream);
-        e != cudaSuccess)
+    if (cudaError_t e = clear_front(h, s, m, stream); e != cudaSuccess)
         return bail(cuda_fail(e, "memset scratch"));
     if (h->checked) {
         B200_STEP(timed(h, "check_csr_A", 0, -1, A->m, stream, [&](cudaStream_t ss) {
@@ -1931,10 +1937,7 @@ spgemm_status transpose(spgemm_handle_s* h, const spgemm_csr_view* A, spgemm_csr
     } while (0)
     Scratch s;
     B200_STEP(ensure_scratch(h, n, &s, stream));
-    B200_CUDA(cudaMemsetAsync(h->scratch, 0,
-                              reinterpret_cast<char*>(s.hist1) - static_cast<char*>(h->scratch),
-                              stream),
-              "memset scratch");
+    B200_CUDA(clear_front(h, s, n, stream), "memset scratch");
     if (h->checked) {
         B200_STEP(timed(h, "check_csr_A", 0, -1, m, stream, [&](cudaStream_t ss) {
             return launch_check_csr(A->rpt, A->col, m, n, nnz, s.status, ss);

@@ -1,11 +1,10 @@
 """GPU: the binning passes at the edges of their ranges.
 
-Row counts around a CTA's rows (256 and 1,024), around the switch between the
-two (148 * 4 * 1,024) and around the largest count that the one-launch passes
-take (2^22), with rows of every fill list's limit and one past it, in one pass
-and in two: every row of A holds one entry, so C's rows are scaled rows of B and
-the comparison is exact.  Then rows of A at the limits of the NIP pass's three
-row classes, against the oracle."""
+Row counts around a CTA's rows (256), a scan tile (1,024) and the largest count
+that the one-launch passes take (2^22), with rows of every fill list's limit
+and one past it, in one pass and in two: every row of A holds one entry, so C's
+rows are scaled rows of B and the comparison is exact.  Then rows of A at the
+limits of the NIP pass's three row classes, against the oracle."""
 import numpy as np
 import pytest
 
@@ -17,7 +16,7 @@ LENGTHS = [0, 1, 12, 13, 48, 49, 192, 193, 512, 513, 768, 769, 1024, 1025, 2048,
 
 
 @pytest.mark.parametrize("passes", [1, 2])
-@pytest.mark.parametrize("m", [1, 255, 256, 257, 1025, 606207, 606208, 4194304, 4194305])
+@pytest.mark.parametrize("m", [1, 255, 256, 257, 1024, 1025, 606208, 4194304, 4194305])
 def test_binning_row_counts(handle, m, passes):
     import torch
 
@@ -58,7 +57,7 @@ def test_nip_row_classes(handle, oracle_mod, passes):
     from gpuspgemm_b200.api import DeviceCSR, proposal
     rng = np.random.default_rng(5)
     k = 5000
-    lens = rng.permutation(np.concatenate([np.repeat([31, 32, 33, 511, 512, 513], 5), [4096, 0],
+    lens = rng.permutation(np.concatenate([np.repeat([31, 32, 33, 127, 128, 129, 513], 5), [4096, 0],
                                            rng.integers(0, 6, 300)]))
     cols = np.concatenate([np.sort(rng.choice(k, x, replace=False)) for x in lens])
     rpt = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
