@@ -484,7 +484,12 @@ __global__ __launch_bounds__(THREADS) void k_esc_warp(ProductArgs p) {
 // (column << SHIFT | q), SHIFT = log2 of the sort capacity (B.n <= 2^(32 -
 // SHIFT)).  The keys are staged in product order and sorted by a stable
 // radix sort of their column bits only (sort.cuh cta_radix_sort: 3 passes
-// for B.n <= 2^21), so a column's products stay in product order.
+// for B.n <= 2^21), so a column's products stay in product order.  The sort
+// takes the row's first column off the keys and no more passes than its span
+// of columns needs: two up to 2^14 columns, one up to 128 (the products of a
+// batch, whose columns lie side by side in B.n; a banded matrix).  20 products,
+// FP32: the 2,048-product kernel 0.349 -> 0.300 ms, the batch 1.162 -> 1.052;
+// rows that span all of B.n pay two reductions (1M power-law unchanged).
 // With WIDE set, columns take more bits than a key has above its product number
 // (B.n > 2^(32 - SHIFT)): the bits above those, at most 7, wait in an array by
 // product number, and the radix sort takes one more pass on them.
@@ -539,6 +544,8 @@ __global__ __launch_bounds__(THREADS) void k_esc_cta(ProductArgs p) {
         copy_scaled_b_row<V>(p, row, p.a_rpt[row], c0, tid, THREADS);
         return;
     }
+    uint32_t* span = reinterpret_cast<uint32_t*>(sc.aux);  // set before the walk's barriers
+    if (tid < 2) span[tid] = tid == 0 ? ~0u : 0u;
     cta_for_products_mlp<THREADS, kWalkU>(
         p.a_col, p.b_rpt, p.a_rpt[row], p.a_rpt[row + 1], sc,
         [&](int qb, int ai, int) {
@@ -557,8 +564,9 @@ __global__ __launch_bounds__(THREADS) void k_esc_cta(ProductArgs p) {
         });
     // the column bits of the keys: B.n - 1 needs this many
     const int colbits = 32 - __clz(p.n_cols > 1 ? p.n_cols - 1 : 1);
-    cta_radix_sort<THREADS, L::RMAX>(keys, nip, SHIFT, min(colbits, L::LOW), hist, sc.warp_tot,
-                                     WIDE ? hi : nullptr, QMASK);
+    const uint32_t first = cta_radix_sort<THREADS, L::RMAX>(
+        keys, nip, SHIFT, min(colbits, L::LOW), hist, sc.warp_tot, WIDE ? hi : nullptr, QMASK,
+        WIDE ? nullptr : span) >> SHIFT;  // 0 if WIDE
     auto column = [&](uint32_t u) -> uint32_t {
         if constexpr (WIDE) return (static_cast<uint32_t>(hi[u & QMASK]) << L::LOW) | (u >> SHIFT);
         else return u >> SHIFT;
@@ -591,7 +599,7 @@ __global__ __launch_bounds__(THREADS) void k_esc_cta(ProductArgs p) {
                 if (column(w) != c) break;
                 sum += vals[w & QMASK];
             }
-            out_col[r] = static_cast<int32_t>(c);
+            out_col[r] = static_cast<int32_t>(first + c);
             out_val[r] = sum;
             r++;
         }

@@ -218,12 +218,16 @@ __device__ __forceinline__ void cta_sort_swz(int32_t* keys, int n) {
 // whose low bits hold their input position come out ordered by the sort bits
 // and then by position.  With `hi` given, one more pass follows on the digits
 // hi[key & hi_mask]: bits above the key's 32, kept beside the keys by their
-// low bits.
+// low bits.  With `span` given ({~0, 0}, set before the caller's last barrier)
+// the first pass also finds the smallest and the largest key, the smallest's
+// sort bits are taken off every key (and returned; the caller adds them back),
+// and only the bits of what is left are sorted, nbits at most.
 template<int THREADS, int RMAX>
-__device__ __forceinline__ void cta_radix_sort(uint32_t* keys, int n, int lo_bit, int nbits,
-                                               int32_t* hist, int32_t* warp_tot,
-                                               const uint8_t* hi = nullptr,
-                                               uint32_t hi_mask = 0u) {
+__device__ __forceinline__ uint32_t cta_radix_sort(uint32_t* keys, int n, int lo_bit, int nbits,
+                                                   int32_t* hist, int32_t* warp_tot,
+                                                   const uint8_t* hi = nullptr,
+                                                   uint32_t hi_mask = 0u,
+                                                   uint32_t* span = nullptr) {
     constexpr int NW = THREADS / kWarp;
     constexpr int DIGITS = 128;
     static_assert(NW * DIGITS == 4 * THREADS, "four counters per thread in the scan");
@@ -234,7 +238,8 @@ __device__ __forceinline__ void cta_radix_sort(uint32_t* keys, int n, int lo_bit
     const int S = kWarp * ((n + THREADS - 1) / THREADS);
     const int R = S / kWarp;  // <= RMAX
     int32_t* wh = hist + w * DIGITS;
-    const int passes = (nbits + 6) / 7;
+    int passes = (nbits + 6) / 7;
+    uint32_t base = 0u;
     for (int pass = 0; pass < passes + (hi != nullptr ? 1 : 0); pass++) {
         const int bit = lo_bit + 7 * pass;
         auto digit = [&](uint32_t key) -> unsigned {
@@ -250,7 +255,31 @@ __device__ __forceinline__ void cta_radix_sort(uint32_t* keys, int n, int lo_bit
         }
 #pragma unroll
         for (int c = 0; c < DIGITS / kWarp; c++) wh[c * kWarp + lane] = 0;
+        if (span != nullptr && pass == 0) {
+            uint32_t least = ~0u;
+            uint32_t most = 0u;
+#pragma unroll
+            for (int i = 0; i < RMAX; i++) {
+                if (i < R && w * S + kWarp * i + lane < n) {
+                    least = min(least, k[i]);
+                    most = max(most, k[i]);
+                }
+            }
+            least = __reduce_min_sync(0xffffffffu, least);
+            most = __reduce_max_sync(0xffffffffu, most);
+            if (lane == 0) {
+                atomicMin(span, least);
+                atomicMax(span + 1, most);
+            }
+        }
         __syncthreads();  // every key is in registers; the counters are clear
+        if (span != nullptr && pass == 0) {
+            base = span[0] >> lo_bit << lo_bit;
+            const uint32_t range = (span[1] - base) >> lo_bit;
+            passes = min(passes, max(1, (32 - __clz(static_cast<int>(range)) + 6) / 7));
+#pragma unroll
+            for (int i = 0; i < RMAX; i++) k[i] -= base;
+        }
 #pragma unroll
         for (int i = 0; i < RMAX; i++) {
             if (i < R) {
@@ -296,6 +325,7 @@ __device__ __forceinline__ void cta_radix_sort(uint32_t* keys, int n, int lo_bit
         }
         __syncthreads();
     }
+    return base;
 }
 
 }  // namespace b200
