@@ -14,7 +14,6 @@
 // creates/destroys its streams and scratch in every call (setup.cuh:164-165,
 // cleanup.cuh:15-31); here streams, events and scratch live in the handle.
 #include <algorithm>
-#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -22,10 +21,12 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/spgemm.h"
 #include "common.cuh"
+#include "host_wait.hpp"
 #include "kernels.hpp"
 
 namespace b200 {
@@ -369,6 +370,17 @@ spgemm_status mirror_finish(spgemm_handle_s* h, const Plan* plan, const Scratch&
     return SPGEMM_OK;
 }
 
+// The driver's own choice for a process with one context is to spin.
+WaitSchedule wait_schedule() {
+    unsigned flags = 0;
+    if (cudaGetDeviceFlags(&flags) != cudaSuccess) return WaitSchedule::kSpin;
+    switch (flags & cudaDeviceScheduleMask) {
+    case cudaDeviceScheduleYield: return WaitSchedule::kYield;
+    case cudaDeviceScheduleBlockingSync: return WaitSchedule::kBlock;
+    default: return WaitSchedule::kSpin;
+    }
+}
+
 // One synchronisation: a one-CTA kernel behind the stream's work writes the
 // scratch front to page-locked memory and raises a flag the host polls.  From
 // the last kernel's end to the host's next launch that takes ~8 us where a
@@ -386,18 +398,20 @@ spgemm_status publish_and_wait(spgemm_handle_s* h, cudaStream_t stream, const Sc
         B200_TRY(cudaStreamSynchronize(stream));
         return SPGEMM_OK;
     }
-    const volatile unsigned long long* flag = h->flag;
-    for (unsigned spins = 1; *flag != seq; spins++) {
-        if ((spins & 0xfffu) != 0u) continue;
-        // every few tens of microseconds: has the stream failed?
-        const cudaError_t e = cudaStreamQuery(stream);
-        if (e == cudaErrorNotReady) continue;
-        if (e != cudaSuccess) return cuda_fail(e, "wait for the stream");
-        if (*flag == seq) break;
-        return fail(SPGEMM_ERR_INTERNAL, "the stream ended without publishing its state");
+    cudaError_t failed = cudaSuccess;
+    auto state = [&](cudaError_t e) {
+        if (e == cudaErrorNotReady) return 0;
+        failed = e;
+        return e == cudaSuccess ? 1 : -1;
+    };
+    switch (wait_for_flag(
+        h->flag, seq, wait_schedule(), [&] { return state(cudaStreamQuery(stream)); },
+        [&] { return state(cudaStreamSynchronize(stream)); }, [] { std::this_thread::yield(); })) {
+    case WaitEnd::kRaised: return SPGEMM_OK;
+    case WaitEnd::kFailed: return cuda_fail(failed, "wait for the stream");
+    case WaitEnd::kNotRaised: break;
     }
-    std::atomic_thread_fence(std::memory_order_acquire);
-    return SPGEMM_OK;
+    return fail(SPGEMM_ERR_INTERNAL, "the stream ended without publishing its state");
 }
 
 spgemm_status sync_mirror(spgemm_handle_s* h, cudaStream_t stream, const Plan* plan,
