@@ -250,6 +250,7 @@ cudaError_t launch_bin_offsets_map(const int32_t* src_hist, int32_t* hist, int32
 // kAppendMaxRows rows: the lists take kListBins words a row.
 constexpr int32_t kAppendMaxRows = int32_t(1) << 22;
 constexpr int kListBins = 12;
+static_assert(kListBins <= kMaxBins, "a list per bin");
 // key = NIP, written to c_rpt; off (or nullptr) receives each row's slot start
 cudaError_t launch_nip_append(const int32_t* a_rpt, const int32_t* a_col, const int32_t* b_rpt,
                               int32_t m, int32_t* c_rpt, int32_t* off, int32_t* lists,

@@ -28,6 +28,7 @@
 #include "common.cuh"
 #include "host_wait.hpp"
 #include "kernels.hpp"
+#include "lists.hpp"
 
 namespace b200 {
 namespace {
@@ -536,48 +537,6 @@ struct CaptureReq {
     cudaGraph_t graph = nullptr;
 };
 
-// Append binning's row lists: bin b's at b * m (the device only counts rows).
-void list_offsets(Plan* plan, int nb, int32_t m) {
-    for (int b = 0; b < nb; b++) plan->bin_off[b] = b * m;
-}
-
-// The limits append binning counts one-pass rows by: the fill ladder's, and,
-// where the fill may expand, sort and compress, kEscSplit, kEscCtaSmall and
-// kEscCtaMid too.  Which kernel takes which list is decided when the sample is
-// known: src[e] is the fill bin limit e comes from (kFromSplit, kFromSmall:
-// inserted).
-constexpr int kFromSplit = -1;
-constexpr int kFromSmall = -2;
-struct ListLadder {
-    Ladder lad;
-    int src[kMaxBins];
-    // the fill bin that list e belongs to
-    int fill_bin(int e, bool split) const {
-        if (src[e] == kFromSplit) return kEscBins - 1;
-        if (src[e] == kFromSmall) return kEscBins;
-        return split && src[e] == kEscBins - 1 ? kEscBins : src[e];
-    }
-};
-
-ListLadder list_ladder(const Ladder& fill, bool esc) {
-    ListLadder l = {};
-    int nb = 0;
-    for (int b = 0; b < fill.nb; b++) {
-        auto put = [&](int32_t limit, int from) {
-            l.lad.limit[nb] = limit;
-            l.src[nb++] = from;
-        };
-        if (esc && b == kEscBins - 1) put(kEscSplit, kFromSplit);
-        if (esc && b == kEscBins) put(kEscCtaSmall, kFromSmall);
-        if (esc && b == kEscBins) put(kEscCtaMid, kFromSmall);
-        put(fill.limit[b], b);
-        // rows forced to bin min_bin or above: to the lists past the bin below
-        if (b == fill.min_bin - 1) l.lad.min_bin = nb;
-    }
-    l.lad.nb = nb;
-    return l;
-}
-
 // Column-window bins take a bin's rows when the sampled rows (two passes: the
 // product) repeat their columns at least kWinMinRatio times -- their walks then
 // cost less than the hash bins' and than sorting every product -- and the
@@ -817,7 +776,9 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
             }
         }
     }
-    const ListLadder lists = list_ladder(ladf, esc_mode != 2);
+    ListLadder lists;
+    if (!list_ladder(ladf, esc_mode != 2, &lists) || nsym > kListBins)
+        return bail(fail(SPGEMM_ERR_INTERNAL, "more fill or count bins than row lists"));
     const bool nip_counts_fill = !append && early && ladx_ok;
     bool mirror_pending = false;  // mirror_start ran: the first wait is on its event
     // (the row pointer's look-back scan runs once per product: its state was
@@ -1976,6 +1937,8 @@ spgemm_status transpose(spgemm_handle_s* h, const spgemm_csr_view* A, spgemm_csr
     const int nctas = bin_ctas(n);
     const bool append = n <= kAppendMaxRows;
     if (append) {
+        if (ntl > kListBins)
+            return bail(fail(SPGEMM_ERR_INTERNAL, "more sort bins than row lists"));
         B200_STEP(timed(h, "tr_scan_bins", 2, -1, n, stream, [&](cudaStream_t ss) {
             return launch_rpt_scan_append(T->rpt, n, s.scan_state, s.plan2, s.status, s.bins2, n,
                                           lad, ss);
