@@ -204,7 +204,9 @@ struct EscSample {
     int64_t row_nip[kEscBins + 1];
     int64_t rows[kEscBins + 1];
     int32_t span[kEscBins + 1];
-    int32_t pad2;
+    // the most columns of a sampled row whose count ended inside a long B row
+    // (an upper bound; 0: no such row): the ratios say little about it
+    int32_t cols[kEscBins + 1];
 };
 constexpr int kSampleMaxNip = 3072;
 cudaError_t launch_esc_sample(const ProductArgs& p, int32_t m, int32_t samples,

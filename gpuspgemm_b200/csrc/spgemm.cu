@@ -1043,8 +1043,8 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
                 const int most = std::min(fil[b].limit, p1.max_key);
                 const double ratio = static_cast<double>(es.all_nip[b]) /
                                      static_cast<double>(es.all_nnz[b]);
-                const int columns =
-                    std::min(most, static_cast<int>(kWinColumnSpare * most / ratio) + 2);
+                const int columns = std::min(
+                    most, std::max(static_cast<int>(kWinColumnSpare * most / ratio) + 2, es.cols[b]));
                 if (ratio >= kThreadMinRatio && columns <= kThreadCap && n <= kThreadCols &&
                     bin_rows[b] >= kThreadRows) {
                     one_fil[b] = thread_fill_bin(sizeof(V));
