@@ -144,6 +144,7 @@ __global__ __launch_bounds__(kNipThreads) void k_nip_hist(
                   static_cast<unsigned long long>(t));
         atomicMax(&plan->max_key, mx);
         if (cta_sum != nullptr) cta_sum[blockIdx.x] = t;
+        if (blockIdx.x == 0) plan->entries = a_rpt[m] - a_rpt[0];
     }
     if (tid < kMaxBins) {
         hist[blockIdx.x * kMaxBins + tid] = s_hist[tid];
@@ -350,6 +351,7 @@ __global__ __launch_bounds__(kBinThreads) void k_nip_append(
         key = INT32_MAX;
     }
     if (r < m) c_rpt[r] = key;
+    if (blockIdx.x == 0 && threadIdx.x == 0) plan->entries = a_rpt[m] - a_rpt[0];
     append_keys(key, nip, row0, m, off, lists, stride, plan, lad);
 }
 

@@ -29,6 +29,7 @@ struct Plan {
     int32_t overflow;         // a sum left int32 range
     int32_t bin_size[kMaxBins];
     int32_t bin_off[kMaxBins];
+    int64_t entries;          // NIP pass: A's entries in these rows (A may be a row range)
 };
 
 // Everything a per-bin kernel needs.  Values are passed as void* and cast by

@@ -884,6 +884,10 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     Plan p1 = h->mirror->plan;  // bin sizes valid once the count binning ran
     h->info.nip = p1.total_key;
     h->info.max_row_nip = p1.max_key;
+    // (A->nnz counts the whole matrix where A is a range of its rows: a batch's
+    // group, a caller's view)
+    const double mean_b_row = static_cast<double>(p1.total_key) /
+                              static_cast<double>(std::max<int64_t>(p1.entries, 1));
     if (append) list_offsets(&p1, nsym, m);
     bool counted = !early;
     if (counted)
@@ -1036,7 +1040,7 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
         // column-window bins where the sampled rows repeat their columns
         bool windows = false;
         if (sampled && h->esc != 2) {
-            const int lanes = win_lanes(static_cast<double>(nip_total) / A->nnz);
+            const int lanes = win_lanes(mean_b_row);
             for (int b = 0; b <= kEscBins; b++) {
                 if ((h->info.esc_mask >> b) & 1) continue;
                 if (es.all_nnz[b] <= 0) continue;
@@ -1260,7 +1264,7 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     // ---- sym1: exact nnz per row --------------------------------------------
     // column-window bins for the team bins' rows where the sampled rows of all
     // classes suit them
-    const int lanes = win_lanes(static_cast<double>(nip_total) / A->nnz);
+    const int lanes = win_lanes(mean_b_row);
     const int windows = sampled && h->esc != 2 ? win_words(es, 0, kEscBins) : 0;
     BinLauncher count_bins[kMaxBins];
     for (int b = 0; b < nsym; b++)
