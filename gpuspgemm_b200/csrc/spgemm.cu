@@ -538,29 +538,70 @@ struct CaptureReq {
 };
 
 // Column-window bins take a bin's rows when the sampled rows (two passes: the
-// product) repeat their columns at least kWinMinRatio times -- their walks then
-// cost less than the hash bins' and than sorting every product -- and the
-// sampled span needs at most kWinMaxWords words and kWinWordsPerNip words per
-// product of a row (the bitmap is cleared and scanned whole).
+// product) repeat their columns at least kWinMinRatio times and the sampled span
+// needs at most kWinMaxWords words, and of these no more per product of a row
+// than the constants below: the bitmap is cleared and scanned whole, which costs
+// about a sixth of a product a word and, past ~900 words, CTAs on the SM.  A walk
+// whose B rows leave lanes of the team idle costs more per product, so the limit
+// is for full teams and shrinks with the lanes in use.
+// Measured (B200, FP64; hash -> window, ms; W the span's words per product, r =
+// NIP / nnz), whole calls:
+//   one pass, 80,000 rows of 300 products, r = 3 (15 of 16 lanes): W 0.7 0.49 ->
+//   0.36, 1.4 0.49 -> 0.45, 2.9 0.48 -> 0.56; 200,000 of 120, r = 6 (10 of 16): W
+//   0.7 0.37 -> 0.37, 1.3 0.37 -> 0.43; 27-point stencil squared (27 of 32) 80^3
+//   (W 1.2) 4.0 -> 3.1, 100^3 (1.7) 7.8 -> 8.2
+//   two passes, the 300-product rows: 0.45 -> 0.37, 0.45 -> 0.46, 0.46 -> 0.61;
+//   fill alone (a plan's replay) 0.26 -> 0.22, 0.26 -> 0.31, 0.27 -> 0.43; stencil
+//   fill 80^3 2.9 -> 2.8, 100^3 5.8 -> 7.8
+// Below a ratio of 1.5 the sample walks a row's first 256 products only and may not
+// know its span; rows of up to 192 products then sort (120 products, r = 1.2: sort
+// 0.32, hash 0.35, window 0.26 where the span is known).
 constexpr double kWinMinRatio = 1.5;
-constexpr double kWinWordsPerNip = 4.0;
-// A thread per row (rows of at most kThreadCap columns) from this ratio on.
+constexpr double kWinOnePassWords = 2.0;
+constexpr double kWinTwoPassWords = 1.65;  // the count
+constexpr double kWinFillWords = 1.5;      // the fill of two passes and of plans
+// Words per lane of a team: past this a narrow team's warp holds so many bitmaps
+// that few warps fit an SM (300,000 rows of 160 products on 12 columns, 4 lanes,
+// 210 words: hash 0.74, window 0.76).
+constexpr int kWinWordsPerLane = 40;
+// Fewer rows than kThreadRows of fewer products than this fill by hashing: the
+// kernels take some 30 us and the window's setup shows (50,000 rows of 24
+// products, r = 1.9: hash 0.030, window 0.035; 400,000 rows 0.158, 0.138).
+constexpr int kWinFewProducts = 32;
+// So do rows that read B rows of fewer entries than this on average (half of the
+// team's four lanes idle), from this many products on: 6,000 rows of 80 products on
+// 18 columns, B rows of two: hash 0.028, window 0.038; 200,000 rows 0.236, 0.261;
+// 6,000 of 34 on 8 columns 0.023, 0.023.  (Wider teams win with half their lanes:
+// 200,000 rows of 300 products on 100 columns, B rows of five on 8 lanes, 0.685 ->
+// 0.630; of 510 on 150, B rows of 17 on 32 lanes, 1.07 -> 0.89.)
+constexpr double kWinNarrowRow = 2.25;
+constexpr int64_t kWinNarrowNip = int64_t(1) << 18;
+// Teams of four lanes hold at most this many columns: eight teams' sums a warp
+// leave little of the SM's memory to L1 (200,000 rows of 180 products, B rows of
+// three, fill alone: on 40 columns hash 0.490, window 0.446; sums for 53 columns
+// 0.469, 0.718; on 60 columns 0.479, 0.722).
+constexpr int kWinNarrowCap = 48;
+// A thread per row (rows of at most kThreadCap columns) from this ratio on (fill
+// alone, hash / window / thread: 65,536 rows of 24 products, ratio 3.1, 0.030 /
+// 0.029 / 0.028; 300,000 rows 0.095 / - / 0.074; of 81 products, ratio 9, 0.27 /
+// 0.19 / 0.16).
 constexpr double kThreadMinRatio = 3.0;
 // What a row may have past the sampled rows' span and past its columns as the
 // sampled ratio estimates them; rows past that go to the fail list.
 constexpr double kWinSpanSpare = 1.1;
 constexpr double kWinColumnSpare = 1.3;
 
-// Lanes per row for B rows of this mean length.
+// Lanes per row for B rows of this mean length, and the share of them at work.
 int win_lanes(double mean) {
     int g = 4;
     while (g < 32 && g < mean) g *= 2;
     return g;
 }
+double win_lane_share(double mean) { return std::min(mean / win_lanes(mean), 1.0); }
 
 // The bitmap's words for the sampled classes [first, last], or 0 when they do
-// not suit the window bins.
-int win_words(const EscSample& es, int first, int last) {
+// not suit the window bins; per_nip: the most words per product of a row.
+int win_words(const EscSample& es, int first, int last, double per_nip, int lanes) {
     int64_t nip = 0, nnz = 0, row_nip = 0, rows = 0;
     int32_t span = 0;
     for (int b = first; b <= last; b++) {
@@ -572,8 +613,8 @@ int win_words(const EscSample& es, int first, int last) {
     }
     if (rows <= 0 || static_cast<double>(nip) < kWinMinRatio * static_cast<double>(nnz)) return 0;
     const double words = std::ceil(kWinSpanSpare * span / 32.0) + 1.0;
-    if (words > kWinMaxWords ||
-        words > kWinWordsPerNip * static_cast<double>(row_nip) / static_cast<double>(rows))
+    if (words > kWinMaxWords || words > kWinWordsPerLane * lanes ||
+        words > per_nip * static_cast<double>(row_nip) / static_cast<double>(rows))
         return 0;
     return static_cast<int>(words);
 }
@@ -1055,8 +1096,9 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
                     windows = true;
                     continue;
                 }
-                const int words = win_words(es, b, b);
-                if (words == 0) continue;
+                const int words =
+                    win_words(es, b, b, kWinOnePassWords * win_lane_share(mean_b_row), lanes);
+                if (words == 0 || (lanes == 4 && columns > kWinNarrowCap)) continue;
                 one_fil[b] = win_fill_bin(sizeof(V), lanes, words, columns);
                 windows = true;
             }
@@ -1265,7 +1307,10 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     // column-window bins for the team bins' rows where the sampled rows of all
     // classes suit them
     const int lanes = win_lanes(mean_b_row);
-    const int windows = sampled && h->esc != 2 ? win_words(es, 0, kEscBins) : 0;
+    const double lane_share = win_lane_share(mean_b_row);
+    const int windows = sampled && h->esc != 2
+                            ? win_words(es, 0, kEscBins, kWinTwoPassWords * lane_share, lanes)
+                            : 0;
     BinLauncher count_bins[kMaxBins];
     for (int b = 0; b < nsym; b++)
         count_bins[b] =
@@ -1400,15 +1445,25 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     BinLauncher two_fil[kMaxBins];
     for (int b = 0; b < nfil; b++) two_fil[b] = fil[b];
     const double repeats = static_cast<double>(nip_total) / static_cast<double>(nnz);
-    const bool fill_windows = windows > 0 && repeats >= kWinMinRatio;
-    if (fill_windows)
+    bool fill_windows = false;
+    if (sampled && h->esc != 2 && repeats >= kWinMinRatio) {
+        const bool few_products = m < kThreadRows && nip_total < int64_t(kWinFewProducts) * m;
+        const bool narrow_rows = mean_b_row < kWinNarrowRow && nip_total >= kWinNarrowNip;
+        const bool by_window =
+            windows > 0 && !few_products && !narrow_rows &&
+            win_words(es, 0, kEscBins, kWinFillWords * lane_share, lanes) > 0;
         for (int b = 0; b <= kEscBins; b++) {
             const int cap = std::min(lad2.limit[b], p2.max_key);
-            two_fil[b] = repeats >= kThreadMinRatio && cap <= kThreadCap && n <= kThreadCols &&
-                                 p2.bin_size[b] >= kThreadRows
-                             ? thread_fill_bin(sizeof(V))
-                             : win_fill_bin(sizeof(V), lanes, windows, cap);
+            if (repeats >= kThreadMinRatio && cap <= kThreadCap && n <= kThreadCols &&
+                p2.bin_size[b] >= kThreadRows)  // (whatever the span)
+                two_fil[b] = thread_fill_bin(sizeof(V));
+            else if (by_window && (lanes > 4 || cap <= kWinNarrowCap))
+                two_fil[b] = win_fill_bin(sizeof(V), lanes, windows, cap);
+            else
+                continue;
+            fill_windows = true;
         }
+    }
     mark(4);
     DevStatus* fill_status = s.status;
     if (cr != nullptr && cr->plan != nullptr) {
