@@ -711,7 +711,8 @@ __device__ __forceinline__ void scan1_tile(int32_t* __restrict__ cnt, int32_t m,
                                            unsigned long long* __restrict__ state,
                                            Plan* __restrict__ plan, DevStatus* __restrict__ st,
                                            int32_t* __restrict__ lists, int64_t stride,
-                                           const Ladder& lad) {    constexpr int NW = kScanThreads / kWarp;
+                                           const Ladder& lad) {
+    constexpr int NW = kScanThreads / kWarp;
     constexpr int PER = TILE / kScanThreads;  // rows per thread
     constexpr unsigned kAll = 0xffffffffu;
     __shared__ int32_t s_row[TILE + TILE / 32];

@@ -1587,10 +1587,10 @@ B200_S2N_BITMAP_LADDER(double)
 B200_S2N_BITMAP_LADDER(float)
 #undef B200_S2N_BITMAP_LADDER
 
-// One-pass ladder for B.n <= kBitmapCols: the smallest rows packed many to a
-// warp (k_esc_warp), the team bins and the 256-thread bin expand, sort and
-// compress (k_esc_team, k_esc_cta) with the hash bins' row limits; the bitmap
-// and global bins are the bitmap ladder's.
+// One-pass ladder: the smallest rows packed many to a warp (k_esc_warp), the
+// team bins and the 256-thread bin expand, sort and compress (k_esc_team,
+// k_esc_cta; B.n <= kEscCols) with the hash bins' row limits; the bitmap and
+// global bins are the bitmap ladder's (B.n <= kBitmapCols).
 template<typename V>
 struct S2nEscLadder {
     static const BinLauncher entries[];

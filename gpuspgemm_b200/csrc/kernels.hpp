@@ -99,9 +99,12 @@ struct BinLauncher {
 // and value, fit this many bytes and the product has at least kOnePassMinNip
 // intermediate products, kOnePassMinNipUnsampled where the compression sample
 // did not run (its rows are then hashed, not sorted).  One pass against two,
-// whole calls, us: power-law FP64 30,000 rows at exponent 2.3 (NIP 192 k) 182
-// against 284, at 2.0 (839 k) 222 against 311; uniform 10,000 x 8 (640 k) 119
-// against 145; power-law 10,000 rows at 2.3 (66 k) 191 against 251.
+// whole calls, FP64, us.  Sampled: power-law 13,000 rows at exponent 2.3 (NIP 89 k)
+// 141 against 236, 8,000 at 2.0 (211 k) 142 / 240, 30,000 at 2.3 (208 k) 144 / 255;
+// uniform 4,500 x 8 (288 k) 80 / 104, 2,000 x 20 (800 k) 105 / 159.  Not sampled,
+// forced: power-law 10,000 at 2.3 (73 k) 192 / 228, 5,000 at 2.0 (112 k) 227 / 228;
+// uniform 1,000 x 8 (64 k) 86 / 96, 4,096 x 8 (262 k) 89 / 99: one pass, hashing
+// too, takes 82-100 % there; the line for it has not been moved.
 constexpr uint64_t kOnePassMaxBytes = uint64_t(4) << 30;
 constexpr int64_t kOnePassMinNip = int64_t(1) << 16;
 constexpr int64_t kOnePassMinNipUnsampled = int64_t(1) << 21;
@@ -120,9 +123,10 @@ int s2n_bitmap_ladder_f32(const BinLauncher** out);
 // Expanding, sorting and compressing packs a column, a product's place and, in
 // the warp bins, a row into one 32-bit key: B.n up to this.
 constexpr int kEscCols = 1 << 22;
-// One-pass ladder for B.n <= kBitmapCols (key = NIP of the row): the warp,
-// team and 256-thread bins expand, sort and compress; then the bitmap ladder's
-// bitmap and global bins.  Same bin count and limits as the bitmap ladder.
+// One-pass ladder (key = NIP of the row): its warp, team and 256-thread bins
+// expand, sort and compress, for B.n <= kEscCols; its last two are the bitmap
+// ladder's bitmap and global bins, for B.n <= kBitmapCols.  Same limits as the
+// bitmap ladder and as the wide ladder's first five bins.
 int s2n_esc_ladder_f64(const BinLauncher** out);
 int s2n_esc_ladder_f32(const BinLauncher** out);
 // The one-pass ladder's largest team bin when its split is kEscSplit
@@ -174,8 +178,8 @@ constexpr double kEscMaxRatio[kEscBins] = {8.0, 8.0, 1.4, 1.1};
 // The one-pass ladder's bins that may expand-sort-compress: the team bins and
 // the 256-thread bin, which follows the sample of the largest team bin.
 constexpr int kEscLadderBins = kEscBins + 1;
-// The sample runs for products with at least this many entries in A (a
-// smaller product's launches cost more than what it decides).
+// The sample runs for products with more than 2^15 entries in A: a smaller
+// product's phases take about as long as the sample, ~20 us.
 constexpr int64_t kSampleMinNnz = (int64_t(1) << 15) + 1;
 // Products with at least this many entries in A are expected to run one pass:
 // they are binned for the fill right after the NIP pass, before the first
@@ -250,7 +254,7 @@ cudaError_t launch_bin_offsets_map(const int32_t* src_hist, int32_t* hist, int32
 // Append binning, one launch a pass (rows into per-bin lists: bin b's rows at
 // lists[b * stride ...], stride >= m, their number in plan->bin_size[b]; the
 // plan zeroed by the caller receives the keys' total and max).  Used up to
-// kAppendMaxRows rows: the lists take kListBins words a row.
+// kAppendMaxRows rows: the lists take kListBins words a row (lists.hpp).
 constexpr int32_t kAppendMaxRows = int32_t(1) << 22;
 constexpr int kListBins = 12;
 static_assert(kListBins <= kMaxBins, "a list per bin");

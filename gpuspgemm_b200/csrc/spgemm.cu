@@ -1,15 +1,20 @@
 // Host orchestration of the B200 CSR SpGEMM and its C ABI (include/spgemm.h).
 //
 // One product (reference: proposal_inner, proposal.cuh:26-80):
-//   count pass      NIP per row -> per-CTA histograms -> offsets -> stable
-//                   scatter of rows into count bins            [host sync 1]
+//   count pass      NIP per row and a row list per bin, in one launch; beside it
+//                   a sample of rows that chooses kernels          [host sync 1]
+//   two passes:
 //   sym1            one kernel per non-empty count bin, heavy bins first,
 //                   spread over side streams; cluster-bin spills go to the
 //                   global bin in stream order (no host round-trip)
-//   scan pass       nnz histograms -> offsets -> scatter + exclusive scan of
-//                   C.rpt                                         [host sync 2]
+//   scan pass       exclusive scan of C.rpt and the fill's row lists, in one
+//                   launch                                         [host sync 2]
 //   fill+numeric    allocate C.col / C.val, one fused kernel per non-empty bin
 //                   [final sync]
+//   one pass (most sampled products): the fill kernels write NIP-sized slots and
+//   each row's nnz, a scan makes C.rpt, a copy packs C
+//   (more than kAppendMaxRows rows: binning takes three launches a pass --
+//   histograms, offsets, stable scatter)
 // The reference synchronises with the host after every binning step and
 // creates/destroys its streams and scratch in every call (setup.cuh:164-165,
 // cleanup.cuh:15-31); here streams, events and scratch live in the handle.
@@ -742,7 +747,7 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     // beside the NIP pass (forked before it), but queued behind it and at low
     // priority: ahead of it, its CTAs took a third of the SMs' threads and the
     // NIP pass ran in two waves (1M rows: both done at 0.115 ms, now at 0.079;
-    // the product 0.977 -> 0.926 ms).  Past kAppendMaxRows rows it also decides
+    // the product 0.98 -> 0.94 ms).  Past kAppendMaxRows rows it also decides
     // the one-pass fill binning's limits on the device.  Its sums come back
     // with the first synchronisation: they choose one pass or two and, per
     // fill bin, the kernel.
@@ -781,7 +786,9 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     // runs only if it turns out two-pass.  Its fill binning scans a copy of
     // the NIP per row, which the NIP pass writes beside C.rpt.
     // (plans replay the two-pass fill; batches run one pass where their small
-    // rows may expand, sort and compress: 20 products, 32 M NIP, FP32, 1.86 -> 1.27 ms)
+    // rows may expand, sort and compress: FP64, 8 products (15 M NIP) 0.93 -> 0.58 ms,
+    // 20 (34 M) 1.73 -> 1.06, 50 (83 M) 4.08 -> 2.59; a server's saturated stream of
+    // small requests 8.4k -> 9.0k products/s)
     const bool may_one_pass =
         h->one_pass != 2 && (cr == nullptr || (cr->plan == nullptr && narrow && h->esc != 2));
     const bool early = may_one_pass && (h->one_pass == 1 || A->nnz >= kEarlyOnePassNnz);
@@ -1925,7 +1932,7 @@ spgemm_status product_host(spgemm_handle_s* h, const spgemm_csr_view* A,
 // ---- CSR transpose -----------------------------------------------------------
 // T = A^T with sorted columns (k_transpose.cu): column counts and ranks, the
 // binning pass with the scan (T.rpt and length bins of T's rows), a scatter of
-// records, then one ordering kernel per non-empty length bin.  One host synchronisation (the bin
+// positions, then one ordering kernel per non-empty length bin.  One host synchronisation (the bin
 // sizes), like each binning pass of a product.
 template<typename V>
 spgemm_status transpose(spgemm_handle_s* h, const spgemm_csr_view* A, spgemm_csr_out* T,

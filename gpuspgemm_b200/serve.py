@@ -68,7 +68,11 @@ class Request:
 class SpgemmServer:
     """Continuous-batching SpGEMM server on one GPU.
 
-    memory_budget: bytes of C bounds that may be in flight at once.
+    memory_budget: bytes of C bounds that may be in flight at once.  The workers'
+                   handles keep memory of their own on top of it: each its
+                   scratch (~70 bytes a row of its largest unit) and the
+                   temporaries of its largest one-pass unit, 4 + value bytes a
+                   product (12 x batch_nip for a batch in FP64), 4 GiB at most.
     max_batch:     most requests packed into one batched product.
     workers:       worker threads (handles), each with its own stream: units
                    of work run side by side on the GPU.

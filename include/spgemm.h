@@ -190,12 +190,18 @@ typedef enum spgemm_option {
      * temporaries -- NIP entries of column and value -- fit 4 GiB, and the
      * sample does not show most of the NIP in rows of more than 768 products
      * whose columns repeat on average 4 times or more (those fill far smaller
-     * tables in two passes); else two.  1: always one pass; 2: always two passes.  Two
-     * passes: the hash count kernels give each row's exact nnz, the fill
-     * writes C in place.  One pass: rows are filled into NIP-sized slots
-     * while their nnz is counted, then compacted into C -- no count kernels,
-     * one more copy of C.  The one-pass temporaries belong to the handle and
-     * are kept for its next products (freed with the handle). */
+     * tables in two passes); else two.  1: always one pass; 2: always two
+     * passes.  A plain batch with B.n <= 2^20 follows the same rule (two passes
+     * with SPGEMM_OPT_ESC = 2); plans and other batches run two passes.  Two
+     * passes: count kernels give each row's exact nnz, the fill writes C in
+     * place.  One pass: rows are filled into NIP-sized slots while their nnz is
+     * counted, then compacted into C -- no count kernels, one more copy of C.
+     * Both hash, or, where a sample shows rows that repeat their columns inside
+     * a narrow window of B, use a bitmap of the row's window or a thread per row
+     * (off with SPGEMM_OPT_ESC = 2).  The one-pass temporaries, up to 4 GiB,
+     * belong to the handle and are kept for its next products (freed with the
+     * handle); its other scratch is ~56 bytes a row of A and a quarter in
+     * reserve (~16 past 2^22 rows). */
     SPGEMM_OPT_ONE_PASS = 8,
     /* One-pass products with B.n <= 2^22: whether the four team fill bins
      * (rows of up to 12, 48, 192 and 768 intermediate products) and the CTA
@@ -204,7 +210,8 @@ typedef enum spgemm_option {
      * product order -- instead of hashing.  0 (default): per bin, when the NIP / nnz of the
      * bin's rows among 2,048 rows sampled from A is at most 8, 8, 1.4 and 1.1
      * (the CTA bins follow the last team bin's sample; products with
-     * A.nnz > 2^15 -- smaller ones hash); 1: always; 2: never.
+     * A.nnz > 2^15 -- smaller ones hash); 1: always; 2: never, and neither the
+     * window nor the thread-per-row kernels: every bin hashes.
      * spgemm_info.esc_mask says which bins did (bits 0-4). */
     SPGEMM_OPT_ESC = 9
 } spgemm_option;
