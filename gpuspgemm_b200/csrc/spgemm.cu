@@ -551,11 +551,11 @@ struct CaptureReq {
 // is for full teams and shrinks with the lanes in use.
 // Measured (B200, FP64; hash -> window, ms; W the span's words per product, r =
 // NIP / nnz), whole calls:
-//   one pass, 80,000 rows of 300 products, r = 3 (15 of 16 lanes): W 0.7 0.49 ->
-//   0.36, 1.4 0.49 -> 0.45, 2.9 0.48 -> 0.56; 200,000 of 120, r = 6 (10 of 16): W
-//   0.7 0.37 -> 0.37, 1.3 0.37 -> 0.43; 27-point stencil squared (27 of 32) 80^3
-//   (W 1.2) 4.0 -> 3.1, 100^3 (1.7) 7.8 -> 8.2
-//   two passes, the 300-product rows: 0.45 -> 0.37, 0.45 -> 0.46, 0.46 -> 0.61;
+//   one pass, 80,000 rows of 300 products, r = 3 (15 of 16 lanes): W 0.7 0.48 ->
+//   0.36, 1.4 0.48 -> 0.45, 2.9 0.48 -> 0.56; 200,000 of 120, r = 6 (10 of 16): W
+//   0.7 0.36 -> 0.37, 1.3 0.36 -> 0.43; 27-point stencil squared (27 of 32) 80^3
+//   (W 1.2) 4.1 -> 3.1, 100^3 (1.7) 7.9 -> 8.2
+//   two passes, the 300-product rows: 0.43 -> 0.37, 0.43 -> 0.46, 0.44 -> 0.61;
 //   fill alone (a plan's replay) 0.26 -> 0.22, 0.26 -> 0.31, 0.27 -> 0.43; stencil
 //   fill 80^3 2.9 -> 2.8, 100^3 5.8 -> 7.8
 // Below a ratio of 1.5 the sample walks a row's first 256 products only and may not
