@@ -652,8 +652,8 @@ spgemm_status plan_alloc(spgemm_plan_s* plan, void** p, size_t bytes, cudaStream
 }
 
 template<typename V>
-spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm_csr_view* B,
-                      spgemm_csr_out* C, cudaStream_t stream, CaptureReq* cr = nullptr) {
+spgemm_status product_once(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm_csr_view* B,
+                           spgemm_csr_out* C, cudaStream_t stream, CaptureReq* cr) {
     if (h == nullptr) return fail(SPGEMM_ERR_INVALID_ARG, "handle is NULL");
     if (C == nullptr) return fail(SPGEMM_ERR_INVALID_ARG, "C is NULL");
     if (spgemm_status st = check_view(A, "A"); st != SPGEMM_OK) return st;
@@ -1565,6 +1565,23 @@ spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm
     resolve_profile(h);
 #undef B200_STEP
     return SPGEMM_OK;
+}
+
+// A product that chose one pass and does not fit the device's memory -- its
+// temporaries, or C beside them -- gives the temporaries back and runs two passes.
+template<typename V>
+spgemm_status product(spgemm_handle_s* h, const spgemm_csr_view* A, const spgemm_csr_view* B,
+                      spgemm_csr_out* C, cudaStream_t stream, CaptureReq* cr = nullptr) {
+    spgemm_status st = product_once<V>(h, A, B, C, stream, cr);
+    if (st != SPGEMM_ERR_OOM || h->one_pass != 0 || h->info.one_pass == 0) return st;
+    (void)cudaGetLastError();  // (the failed call has waited for its work and freed C)
+    if (h->onepass != nullptr) B200_TRY(cudaFreeAsync(h->onepass, stream));
+    h->onepass = nullptr;
+    h->onepass_bytes = 0;
+    h->one_pass = 2;
+    st = product_once<V>(h, A, B, C, stream, cr);
+    h->one_pass = 0;
+    return st;
 }
 
 // ---- batched products -------------------------------------------------------

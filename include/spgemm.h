@@ -190,7 +190,8 @@ typedef enum spgemm_option {
      * temporaries -- NIP entries of column and value -- fit 4 GiB, and the
      * sample does not show most of the NIP in rows of more than 768 products
      * whose columns repeat on average 4 times or more (those fill far smaller
-     * tables in two passes); else two.  1: always one pass; 2: always two
+     * tables in two passes); else two, and two where the temporaries or C beside
+     * them do not fit the free memory.  1: always one pass; 2: always two
      * passes.  A plain batch with B.n <= 2^20 follows the same rule (two passes
      * with SPGEMM_OPT_ESC = 2); plans and other batches run two passes.  Two
      * passes: count kernels give each row's exact nnz, the fill writes C in

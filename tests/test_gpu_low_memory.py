@@ -1,0 +1,79 @@
+"""GPU: a product or a batch whose one-pass temporaries, or C beside them, do not
+fit the memory that is free runs two passes, with the same C.  In a process of its
+own, which first runs the call with room (one pass) and then takes most of the
+device's free memory."""
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+CHILD = """
+import sys
+sys.path.insert(0, sys.argv[1])
+kind, room = sys.argv[2], int(sys.argv[3]) << 20
+import torch
+from gpuspgemm_b200 import _native as N
+from gpuspgemm_b200.api import DeviceCSR, Handle, PackedBatch, batch, proposal
+import numpy as np
+g = torch.Generator(device="cuda"); g.manual_seed(1)
+m, a_len, b_len, width, groups, per = 700_000, 12, 12, 90, 20, 240
+def stratified(rows, base, parts, span):
+    lo = torch.arange(parts, device="cuda") * span // parts
+    hi = (torch.arange(parts, device="cuda") + 1) * span // parts
+    r = torch.randint(0, 1 << 30, (rows, parts), device="cuda", generator=g)
+    return (base[:, None] + lo + r % (hi - lo)).int().reshape(-1).contiguous()
+nb = groups * per
+bc = stratified(nb, torch.arange(nb, device="cuda") // per * width, b_len, width)
+ac = stratified(m, torch.randint(0, groups, (m,), device="cuda", generator=g) * per, a_len, per)
+val = lambda n: torch.rand(n, device="cuda", generator=g, dtype=torch.float64) - 0.5
+A = DeviceCSR(m, nb, torch.arange(m + 1, device="cuda", dtype=torch.int32) * a_len, ac, val(ac.numel()))
+B = DeviceCSR(nb, groups * width, torch.arange(nb + 1, device="cuda", dtype=torch.int32) * b_len, bc,
+              val(bc.numel()))
+off = lambda *x: np.array(x, np.int32)
+pb = PackedBatch(off(0, m), off(0, nb), off(0, groups * width), A, B)
+def run(h):
+    return batch(pb, h)[0] if kind == "batch" else proposal(A, B, h)
+def digest(C):
+    w = torch.arange(C.nnz, device="cuda", dtype=torch.int64) % 1009 + 1
+    a = int((C.col.long() * w).sum()); del w
+    return C.nnz, int(C.rpt.long().sum()), a, float(C.val.sum())
+h = Handle(0)
+h.set_option(N.OPT_ONE_PASS, 2)   # (its kernels are loaded while there is room)
+C = run(h); del C
+h.set_option(N.OPT_ONE_PASS, 0)
+C = run(h)
+nip = 144 * m
+assert h.info()["nip"] == nip and C.nnz * 2 < nip * 1.25 and 12 * C.nnz < 12 * nip * 0.62
+want = digest(C); del C
+h.close()                         # the last handle: the pool gives its memory back
+torch.cuda.synchronize(); torch.cuda.empty_cache()
+h = Handle(0)
+small = DeviceCSR(100, nb, A.rpt[:101], A.col, A.val)
+proposal(small, B, h)
+free = torch.cuda.mem_get_info()[0]
+take = torch.empty(free - room, dtype=torch.uint8, device="cuda")
+C = run(h)
+if kind == "product":
+    assert h.info()["one_pass"] == 0, h.info()
+del take; torch.cuda.empty_cache()
+got = digest(C)
+assert got[:3] == want[:3] and abs(got[3] - want[3]) <= 1e-6 * C.nnz ** 0.5, (got, want)
+C = run(h)                        # and with room again, one pass
+if kind == "product":
+    assert h.info()["one_pass"] == 1
+print("OK")
+"""
+
+
+# temporaries 1.21 GB, C 0.6-0.75 GB: neither the temporaries fit (1,100 MiB), or C
+# beside them (1,500 MiB)
+@pytest.mark.parametrize("room", [1100, 1500])
+@pytest.mark.parametrize("kind", ["product", "batch"])
+def test_two_passes_when_one_does_not_fit(native_lib, kind, room):
+    root = str(Path(__file__).resolve().parent.parent)
+    res = subprocess.run([sys.executable, "-c", CHILD, root, kind, str(room)],
+                         capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0 and "OK" in res.stdout, res.stderr[-2000:]
