@@ -64,6 +64,7 @@ constexpr size_t kFrontBytes = 4096;
 constexpr int64_t kBitmapBudget = int64_t(1) << 30;
 
 struct Scratch {
+    bool append;  // the row lists of append binning are there
     DevStatus* status;
     Plan* plan1;
     // the row pointer's look-back: a ticket counter and one state per tile
@@ -194,7 +195,9 @@ spgemm_status regrow(spgemm_handle_s* h, void** buf, size_t* have, size_t need,
     return SPGEMM_OK;
 }
 
-spgemm_status ensure_scratch(spgemm_handle_s* h, int32_t m, Scratch* s, cudaStream_t stream) {
+// `append`: with the row lists of append binning (up to kAppendMaxRows rows).
+spgemm_status layout_scratch(spgemm_handle_s* h, int32_t m, bool append, Scratch* s,
+                             cudaStream_t stream) {
     const size_t nctas = static_cast<size_t>(bin_ctas(m > 0 ? m : 1));
     const size_t mm = static_cast<size_t>(m > 0 ? m : 1);
     size_t off = 0;
@@ -217,7 +220,6 @@ spgemm_status ensure_scratch(spgemm_handle_s* h, int32_t m, Scratch* s, cudaStre
     const size_t o_sum = take(sizeof(int64_t) * nctas);
     // append binning: one region of per-bin lists serves the passes in turn
     // (each pass's lists are read before the next pass starts)
-    const bool append = m <= kAppendMaxRows;
     const size_t o_bins1 = take(sizeof(int32_t) * mm * (append ? kListBins : 1));
     const size_t o_bins2 = append ? o_bins1 : take(sizeof(int32_t) * mm);
     const size_t o_fail = take(sizeof(int32_t) * mm);
@@ -227,6 +229,7 @@ spgemm_status ensure_scratch(spgemm_handle_s* h, int32_t m, Scratch* s, cudaStre
         st != SPGEMM_OK)
         return st;
     char* b = static_cast<char*>(h->scratch);
+    s->append = append;
     s->status = reinterpret_cast<DevStatus*>(b + o_status);
     s->plan1 = reinterpret_cast<Plan*>(b + o_plan1);
     s->plan2 = reinterpret_cast<Plan*>(b + o_plan2);
@@ -245,6 +248,15 @@ spgemm_status ensure_scratch(spgemm_handle_s* h, int32_t m, Scratch* s, cudaStre
     s->work = reinterpret_cast<int32_t*>(b + o_work);
     s->scan_state = reinterpret_cast<unsigned long long*>(b + o_scan);
     return SPGEMM_OK;
+}
+
+// The scratch of a product or transpose of m binned rows.  Where the row lists (48
+// bytes a row) do not fit the device's free memory, that of the three-launch binning.
+spgemm_status ensure_scratch(spgemm_handle_s* h, int32_t m, Scratch* s, cudaStream_t stream) {
+    const spgemm_status st = layout_scratch(h, m, m <= kAppendMaxRows, s, stream);
+    if (st != SPGEMM_ERR_OOM || m > kAppendMaxRows) return st;
+    (void)cudaGetLastError();
+    return layout_scratch(h, m, false, s, stream);
 }
 
 // Clears the scratch front and, behind it, the row-pointer scan's state as far
@@ -741,7 +753,7 @@ spgemm_status product_once(spgemm_handle_s* h, const spgemm_csr_view* A, const s
     // ---- count pass: NIP per row and bins ---------------------------------
     const int nctas = bin_ctas(m);
     // one launch per binning pass, a row list per bin (k_bin.cu)
-    const bool append = m <= kAppendMaxRows;
+    const bool append = s.append;
     const Ladder lad1 = make_ladder(sym, nsym, h->min_sym_bin);
     // Compression sample: it reads A and B only, so it runs on a side stream
     // beside the NIP pass (forked before it), but queued behind it and at low
@@ -2018,7 +2030,7 @@ spgemm_status transpose(spgemm_handle_s* h, const spgemm_csr_view* A, spgemm_csr
     }));
     const Ladder lad = make_ladder(tl, ntl, h->min_tr_bin);
     const int nctas = bin_ctas(n);
-    const bool append = n <= kAppendMaxRows;
+    const bool append = s.append;
     if (append) {
         if (ntl > kListBins)
             return bail(fail(SPGEMM_ERR_INTERNAL, "more sort bins than row lists"));

@@ -77,3 +77,57 @@ def test_two_passes_when_one_does_not_fit(native_lib, kind, room):
     res = subprocess.run([sys.executable, "-c", CHILD, root, kind, str(room)],
                          capture_output=True, text=True, timeout=300)
     assert res.returncode == 0 and "OK" in res.stdout, res.stderr[-2000:]
+
+
+LISTS = """
+import sys
+sys.path.insert(0, sys.argv[1])
+import torch
+from gpuspgemm_b200 import _native as N
+from gpuspgemm_b200.api import DeviceCSR, Handle, proposal, transpose
+g = torch.Generator(device="cuda"); g.manual_seed(2)
+m, k, n, used = 4_100_000, 3000, 5000, 82_000
+length = torch.zeros(m, dtype=torch.int64, device="cuda")
+length[torch.arange(used, device="cuda") * (m // used)] = torch.randint(1, 4, (used,), device="cuda",
+                                                                        generator=g)
+rpt = torch.zeros(m + 1, dtype=torch.int64, device="cuda"); rpt[1:] = length.cumsum(0)
+nnz = int(rpt[-1])
+row = torch.repeat_interleave(torch.arange(m, device="cuda"), length)
+at = torch.arange(nnz, device="cuda") - rpt[row]      # an entry's place in its row
+col = at * 1000 + torch.randint(0, 1000, (nnz,), device="cuda", generator=g)
+val = lambda x: torch.rand(x, device="cuda", generator=g, dtype=torch.float64) + 0.5
+A = DeviceCSR(m, k, rpt.int(), col.int(), val(nnz))
+bc = (torch.arange(5, device="cuda") * 1000 + torch.randint(0, 1000, (k, 5), device="cuda",
+                                                            generator=g)).int().reshape(-1).contiguous()
+B = DeviceCSR(k, n, torch.arange(k + 1, device="cuda", dtype=torch.int32) * 5, bc, val(5 * k))
+def run(h):
+    C = proposal(A, B, h); names = {x["name"] for x in h.profile()}
+    R = transpose(DeviceCSR(k, m, tr.rpt, tr.col, tr.val), h)   # A again: m rows
+    return C, R, names | {x["name"] for x in h.profile()}
+h = Handle(0); h.set_option(N.OPT_PROFILE, 1)
+tr = transpose(A, h)
+C0, R0, names = run(h)
+assert "nip_hist" in names and not any(x in names for x in ("nip_fill_scatter", "tr_hist")), names
+assert torch.equal(R0.rpt, A.rpt) and torch.equal(R0.col, A.col) and torch.equal(R0.val, A.val)
+h.close()
+del length, rpt, row, at, col
+torch.cuda.synchronize(); torch.cuda.empty_cache()
+h = Handle(0); h.set_option(N.OPT_PROFILE, 1)
+proposal(DeviceCSR(100, k, A.rpt[:101], A.col, A.val), B, h)
+take = torch.empty(torch.cuda.mem_get_info()[0] - (220 << 20), dtype=torch.uint8, device="cuda")
+C, R, names = run(h)
+assert {"nip_fill_scatter", "tr_hist"} <= names, names
+del take; torch.cuda.empty_cache()
+for X, Y in ((C, C0), (R, R0)):
+    assert torch.equal(X.rpt, Y.rpt) and torch.equal(X.col, Y.col)
+    assert torch.allclose(X.val, Y.val, rtol=1e-14, atol=0)
+print("OK")
+"""
+
+
+# the row lists take 287 MB with their reserve, the other binning's scratch 83 MB
+def test_binning_when_the_row_lists_do_not_fit(native_lib):
+    root = str(Path(__file__).resolve().parent.parent)
+    res = subprocess.run([sys.executable, "-c", LISTS, root], capture_output=True, text=True,
+                         timeout=300)
+    assert res.returncode == 0 and "OK" in res.stdout, res.stderr[-2000:]
